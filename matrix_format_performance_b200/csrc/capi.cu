@@ -211,9 +211,20 @@ namespace {
 // warp tile, the head and tail partial sums (8 bytes each, FP64-sized), the
 // flags and the tail row.  Every call rewrites what it reads: no
 // initialisation.
+size_t carry_ws_bytes(uint64_t warp_tiles) { return sizeof(d::coo_ws_header) + warp_tiles * 24u; }
 size_t coo_ws_bytes(uint32_t nnz) {
-  const uint64_t wt = (nnz + (uint64_t)d::kWarpTile - 1) / d::kWarpTile;
-  return sizeof(d::coo_ws_header) + wt * 24u;
+  return carry_ws_bytes((nnz + (uint64_t)d::kWarpTile - 1) / d::kWarpTile);
+}
+// The per-tile arrays of such a workspace, after its header.
+template <typename T>
+d::coo_carry<T> carries(void *ws, uint32_t warp_tiles) {
+  unsigned char *base = static_cast<unsigned char *>(ws) + sizeof(d::coo_ws_header);
+  d::coo_carry<T> cw;
+  cw.head = reinterpret_cast<T *>(base);
+  cw.tail = reinterpret_cast<T *>(base + (size_t)warp_tiles * 8u);
+  cw.flags = reinterpret_cast<uint32_t *>(base + (size_t)warp_tiles * 16u);
+  cw.tail_row = cw.flags + warp_tiles;
+  return cw;
 }
 constexpr uint32_t kDefaultLong = 4096;
 constexpr uint32_t kDefaultAssist = 64;
@@ -726,12 +737,7 @@ int coo_spmv(uint32_t rows, uint32_t nnz, const T *data, const uint32_t *cols, c
   if (!aligned16(ws)) return fail(MFP_ERROR_INVALID_VALUE, "COO workspace must be 16-byte aligned");
   const uint32_t n_wt = ceil_div(nnz, d::kWarpTile);
   auto *hdr = static_cast<d::coo_ws_header *>(ws);
-  unsigned char *base = static_cast<unsigned char *>(ws) + sizeof(d::coo_ws_header);
-  d::coo_carry<T> cw;
-  cw.head = reinterpret_cast<T *>(base);
-  cw.tail = reinterpret_cast<T *>(base + (size_t)n_wt * 8u);
-  cw.flags = reinterpret_cast<uint32_t *>(base + (size_t)n_wt * 16u);
-  cw.tail_row = cw.flags + n_wt;
+  const d::coo_carry<T> cw = carries<T>(ws, n_wt);
   const uint32_t grid = ceil_div(n_wt, d::kBlock / 32u);
   const int vec = vec_level(data, cols, rids);
   cudaStream_t s = as_stream(stream);
@@ -773,12 +779,7 @@ int csr_tile_spmv(const mfp_csr_plan *plan, const T *data, const uint32_t *cols,
   const uint32_t nnz = plan->nnz, rows = plan->rows;
   const uint32_t n_wt = ceil_div(nnz, d::kWarpTile);
   auto *hdr = static_cast<d::coo_ws_header *>(plan->tile_ws);
-  unsigned char *base = static_cast<unsigned char *>(plan->tile_ws) + sizeof(d::coo_ws_header);
-  d::coo_carry<T> cw;
-  cw.head = reinterpret_cast<T *>(base);
-  cw.tail = reinterpret_cast<T *>(base + (size_t)n_wt * 8u);
-  cw.flags = reinterpret_cast<uint32_t *>(base + (size_t)n_wt * 16u);
-  cw.tail_row = cw.flags + n_wt;
+  const d::coo_carry<T> cw = carries<T>(plan->tile_ws, n_wt);
   const uint32_t grid = ceil_div(n_wt, d::kBlock / 32u);
   const int vec = vec_level(data, cols);
   // 64 row starts per round trip below a mean row length of 8 (power-law 4M
@@ -857,6 +858,29 @@ int scoo_spmv(uint32_t rows, uint32_t slices, uint32_t slice, const T *v, const 
   }
   if (win) return scoo_launch<T, 0, true>(slices, dyn, s, rows, slice, v, ci, ri, sp, win, maxw, order, x, y);
   return scoo_launch<T, 0, false>(slices, dyn, s, rows, slice, v, ci, ri, sp, win, maxw, order, x, y);
+}
+
+// Row-ordered SCOO handles: the slices' warp tiles, then the fix-up.
+template <typename T>
+int scoo_tile_spmv(uint32_t rows, uint32_t slice, uint32_t n_tiles, const d::scoo_tile *tiles, const T *v,
+                   const uint32_t *ci, const uint32_t *ri, const uint16_t *rel, const T *x, T *y, void *ws,
+                   void *stream) {
+  if (rows == 0) return ok();
+  if (!y || !x) return fail(MFP_ERROR_INVALID_VALUE, "null device array");
+  const d::coo_carry<T> cw = carries<T>(ws, n_tiles);
+  const int vec = vec_level(v, ci, ri);
+  const bool r16 = rel && vec == 2 && aligned16(rel);
+  auto k = r16 ? d::scoo_tile_kernel<T, 2, true>
+               : vec == 2 ? d::scoo_tile_kernel<T, 2, false>
+                          : vec == 1 ? d::scoo_tile_kernel<T, 1, false> : d::scoo_tile_kernel<T, 0, false>;
+  cudaStream_t s = as_stream(stream);
+  k<<<ceil_div(n_tiles, d::kBlock / 32u), d::kBlock, 0, s>>>(rows, slice, n_tiles, (const uint4 *)tiles, v, ci, ri,
+                                                             rel, x, y, cw);
+  cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) return cuda_fail(e, "scoo_tile_kernel launch");
+  e = launch_after(d::scoo_fixup_kernel<T>, ceil_div(n_tiles, d::kBlock), s, n_tiles, rows, cw, y);
+  if (e != cudaSuccess) return cuda_fail(e, "scoo_fixup_kernel launch");
+  return ok();
 }
 
 // Pipelined reduced-precision kernel: CAP elements per stage, S stages.  A
@@ -1243,6 +1267,8 @@ struct mfp_matrix {
   uint16_t *delta = nullptr;          // 16-bit column deltas (else cols_a)
   uint32_t *base = nullptr;
   bool rows_unsorted = false;         // SCOO in the sort_cols layout
+  d::scoo_tile *tiles = nullptr;      // row-ordered SCOO: the slices' warp tiles (their carries in ws)
+  uint32_t n_tiles = 0;
   bool long_rows = false;             // reduced-precision CSR: a row longer than kLowpTmaMaxRow
 };
 
@@ -1379,7 +1405,11 @@ int scoo_attach_windows(mfp_matrix *m, const std::vector<uint32_t> &win, const u
   if (!widths.empty()) {
     std::sort(widths.begin(), widths.end());
     const uint32_t p90 = widths[(widths.size() * 9) / 10];
-    if (p90 <= cap) {
+    uint64_t sum = 0;
+    for (uint32_t w : widths) sum += w;
+    // staging pays when each staged entry is read about twice (5-point 1400^2
+    // grid, FP64: 0.8 reads per entry; staging 80 us, gathering 50)
+    if (p90 <= cap && m->nnz >= 2 * sum) {
       use_win = true;
       m->max_window = std::min(cap, widths.back());
       m->max_window = (m->max_window + 3u) & ~3u;
@@ -1391,6 +1421,57 @@ int scoo_attach_windows(mfp_matrix *m, const std::vector<uint32_t> &win, const u
   if ((st = mfp_scoo_slice_order(m->slices, sp_host, order.data())) ||
       (st = track_upload(m, &m->order, order.data(), order.size())))
     return st;
+  return MFP_SUCCESS;
+}
+
+// Whether a row-ordered SCOO handle runs its slices' warp tiles as independent
+// warps (scoo_tile_kernel) instead of one CTA per slice (scoo_kernel):
+//  - when the heaviest slice holds more than twice the mean, which that
+//    slice's CTA would work through alone (B200: power-law, 50k rows FP32 49.7
+//    -> 13.7 us, 1M rows FP64 107 -> 59 us, 4M rows FP32 184 -> 170 us);
+//  - when there is work for the whole chip, and the slices are fewer than the
+//    148 x 6 CTAs it holds or so short (under 16 tiles) that their CTA's
+//    rounds of 8 tiles, barriers and x window weigh (27-point 40^3, 148
+//    slices, FP32 17.8 -> 12.1 us; 5-point 1400^2 FP64, 10 tiles each, 79.8 ->
+//    49.9 us; 1000^2 FP32 27.2 -> 22.6 us).
+// Long balanced slices stay with the one launch (27-point 128^3 122 us against
+// 139, banded 2M rows 118 against 128: no tile table to wait for), and so do
+// small matrices, where the second launch costs more than it gives (64 x 64
+// Laplacian 8.4 us against 11.1).
+bool scoo_use_tiles(const mfp_matrix *m, const uint32_t *sp_host) {
+  if (m->rows_unsorted || m->nnz == 0) return false;
+  uint64_t heaviest = 0, used = 0;
+  for (uint32_t s = 0; s < m->slices && (uint64_t)s * m->slice_size < m->rows; ++s, ++used)
+    if (sp_host[s + 1] > sp_host[s]) heaviest = std::max<uint64_t>(heaviest, sp_host[s + 1] - sp_host[s]);
+  const uint64_t mean = m->nnz / std::max<uint64_t>(1, used);
+  if (heaviest > 2 * mean && heaviest > 16 * d::kWarpTile) return true;
+  return (used < 148u * 6u || mean < 16 * d::kWarpTile) && m->nnz >= 148u * 6u * d::kWarpTile * 4u;
+}
+
+// Row-ordered SCOO: every slice's 256-element tiles (an entry without elements
+// for an empty slice, whose rows it zeroes) and the workspace of their carries.
+int scoo_attach_tiles(mfp_matrix *m, const uint32_t *sp_host) {
+  std::vector<d::scoo_tile> t;
+  t.reserve((size_t)m->nnz / d::kWarpTile + m->slices);
+  for (uint32_t s = 0; s < m->slices && (uint64_t)s * m->slice_size < m->rows; ++s) {
+    const uint32_t eb = sp_host[s], ee = sp_host[s + 1];
+    if (eb >= ee) {
+      t.push_back({0u, 0u, s, d::kSliceEmpty});
+      continue;
+    }
+    for (uint32_t g0 = eb & ~7u; g0 < ee;) {
+      const uint32_t c1 = ee - g0 > d::kWarpTile ? g0 + d::kWarpTile : ee;
+      const bool first = g0 <= eb;
+      t.push_back({g0, c1, s, (first ? (eb - g0) | d::kSliceFirst : 0u) | (c1 == ee ? d::kSliceLast : 0u)});
+      g0 = c1;
+    }
+  }
+  m->n_tiles = (uint32_t)t.size();
+  m->ws_bytes = carry_ws_bytes(m->n_tiles);
+  unsigned char *ws = nullptr;
+  int st;
+  if ((st = track_upload(m, &m->tiles, t.data(), t.size())) || (st = track(m, &ws, m->ws_bytes))) return st;
+  m->ws = ws;
   return MFP_SUCCESS;
 }
 
@@ -1551,12 +1632,13 @@ int mfp_matrix_create_scoo(int vt, uint32_t rows, uint32_t cols, uint32_t nnz, c
   m->slice_size = prm->slice_size;
   m->rows_unsorted = rows_unsorted;
   m->format_bytes = (uint64_t)nnz * (vs + 8) + ((uint64_t)m->slices + 1) * 4 + (uint64_t)cols * vs + (uint64_t)rows * vs;
-  std::vector<uint32_t> win(2 * (size_t)m->slices);
-  mfp_scoo_x_windows(nnz, ci, sp, m->slices, win.data());
+  const bool tiled = scoo_use_tiles(m, sp);
+  std::vector<uint32_t> win(tiled ? 0u : 2 * (size_t)m->slices);  // the tile path gathers x from memory
+  if (!tiled) mfp_scoo_x_windows(nnz, ci, sp, m->slices, win.data());
   int st;
   if ((st = track_upload_bytes(m, &m->vals, v, (size_t)nnz * vs)) || (st = track_upload(m, &m->cols_a, ci, nnz)) ||
       (st = track_upload(m, &m->rows_a, ri, nnz)) || (st = track_upload(m, &m->aux, sp, (size_t)m->slices + 1)) ||
-      (st = scoo_attach_windows(m, win, sp))) {
+      (st = tiled ? scoo_attach_tiles(m, sp) : scoo_attach_windows(m, win, sp))) {
     mfp_matrix_destroy(m);
     return st;
   }
@@ -1722,20 +1804,26 @@ int mfp_matrix_create_device(int format, int vt, uint32_t rows, uint32_t cols, u
       uint32_t *dwin = nullptr;
       if ((st = track_bytes(m, &m->vals, (size_t)nnz * vs)) ||
           (st = track(m, &m->cols_a, nnz)) || (st = track(m, &m->rows_a, nnz)) ||
-          (st = track(m, &m->aux, (size_t)m->slices + 1)) || (st = dmalloc(&dwin, 2 * (size_t)m->slices)))
+          (st = track(m, &m->aux, (size_t)m->slices + 1)))
         return bail(st);
-      std::vector<uint32_t> win(2 * (size_t)m->slices), hsp((size_t)m->slices + 1);
+      std::vector<uint32_t> win, hsp((size_t)m->slices + 1);
       st = mfp_dev_scoo_from_csr(vt, rows, nnz, rp, ci, data, &prm, m->vals, m->cols_a, m->rows_a, m->aux, nullptr);
       if (!st && o.scoo_sort_cols && nnz) {
         st = mfp_dev_scoo_sort_cols(vt, rows, cols, prm.slice_size, nnz, m->vals, m->cols_a, m->rows_a, nullptr);
         m->rows_unsorted = true;
       }
-      if (!st) st = mfp_dev_scoo_x_windows(nnz, m->cols_a, m->aux, m->slices, dwin, nullptr);
-      if (!st && (cudaMemcpy(win.data(), dwin, win.size() * 4, cudaMemcpyDeviceToHost) != cudaSuccess ||
-                  cudaMemcpy(hsp.data(), m->aux, hsp.size() * 4, cudaMemcpyDeviceToHost) != cudaSuccess))
+      if (!st && cudaMemcpy(hsp.data(), m->aux, hsp.size() * 4, cudaMemcpyDeviceToHost) != cudaSuccess)
         st = fail(MFP_ERROR_CUDA, "cudaMemcpy SCOO metadata");
-      cudaFree(dwin);
-      if (st || (st = scoo_attach_windows(m, win, hsp.data()))) return bail(st);
+      const bool tiled = !st && scoo_use_tiles(m, hsp.data());
+      if (!st && !tiled && !(st = dmalloc(&dwin, 2 * (size_t)m->slices))) {
+        win.resize(2 * (size_t)m->slices);
+        st = mfp_dev_scoo_x_windows(nnz, m->cols_a, m->aux, m->slices, dwin, nullptr);
+        if (!st && cudaMemcpy(win.data(), dwin, win.size() * 4, cudaMemcpyDeviceToHost) != cudaSuccess)
+          st = fail(MFP_ERROR_CUDA, "cudaMemcpy SCOO metadata");
+        cudaFree(dwin);
+      }
+      if (st || (st = tiled ? scoo_attach_tiles(m, hsp.data()) : scoo_attach_windows(m, win, hsp.data())))
+        return bail(st);
       break;
     }
     default:
@@ -1846,7 +1934,7 @@ int mfp_matrix_get_info(const mfp_matrix *m, mfp_matrix_info *out) {
     out->kernel_launches = m->nnz ? 2u : (m->rows ? 1u : 0u);
   else if (m->format == MFP_FORMAT_HYBRID)
     out->kernel_launches = 1u + (m->coo_nnz ? (m->coo_nnz > d::kWarpTile ? 2u : 1u) : 0u);
-  else if (m->plan && m->plan->tile)  // CSR vector on short rows: warp pass + fix-up
+  else if ((m->plan && m->plan->tile) || (m->tiles && m->rows))  // warp-tile CSR, row-ordered SCOO: tiles + fix-up
     out->kernel_launches = 2u;
   else
     out->kernel_launches = 1u;
@@ -1884,6 +1972,11 @@ int mfp_matrix_spmv(const mfp_matrix *m, const void *x, void *y, void *stream) {
                    : scoo_spmv<float, true>(m->rows, m->slices, m->slice_size, (const float *)m->vals, m->cols_a,
                                             m->rows_a, m->aux, m->win, m->max_window, m->order, (const float *)x,
                                             (float *)y, stream);
+      if (m->tiles)
+        return f64 ? scoo_tile_spmv<double>(m->rows, m->slice_size, m->n_tiles, m->tiles, (const double *)m->vals,
+                                            m->cols_a, m->rows_a, m->rel, (const double *)x, (double *)y, m->ws, stream)
+                   : scoo_tile_spmv<float>(m->rows, m->slice_size, m->n_tiles, m->tiles, (const float *)m->vals,
+                                           m->cols_a, m->rows_a, m->rel, (const float *)x, (float *)y, m->ws, stream);
       return f64 ? scoo_spmv<double>(m->rows, m->slices, m->slice_size, (const double *)m->vals, m->cols_a,
                                      m->rows_a, m->aux, m->win, m->max_window, m->order, (const double *)x,
                                      (double *)y, stream, m->rel)
@@ -1920,7 +2013,7 @@ static bool writes_y_in_row_order(const mfp_matrix *m) {
     case MFP_FORMAT_SCOO:
     case MFP_FORMAT_CSR_LOWP:
     case MFP_FORMAT_ELL_LOWP:
-      return !(m->plan && m->plan->tile) && !m->rows_unsorted;
+      return !(m->plan && m->plan->tile) && !m->rows_unsorted && !m->tiles;
     case MFP_FORMAT_CSR_VECTOR:
       return !(m->plan && m->plan->tile);
     default:  // COO and the warp-tile kernels write rows as their tiles finish; the hybrid adds into y

@@ -1080,11 +1080,16 @@ __device__ __forceinline__ void coo_put(T *y, uint32_t n_rows, uint32_t row, T v
 // group starting at g0 + 8 l, the lane's cnt products pr and rows rw in hand
 // (rows non-decreasing); prv / nxt are the rows of the elements just before
 // and after the tile (kNoRow at the ends).
-template <typename T, bool ACCUM>
+//
+// SLICE: the tile belongs to a slice of n_rows rows starting at row0 (rw, prv
+// and nxt are slice-local, y is the slice's part of y, kNoRow marks the
+// slice's ends): the slice's empty first and last rows are zeroed here by the
+// whole warp, and the carry records the matrix row.
+template <typename T, bool ACCUM, bool SLICE = false>
 __device__ __forceinline__ void warp_tile_reduce(uint32_t wt, uint32_t g0, uint32_t c1, uint32_t nnz,
                                                  uint32_t n_rows, const T (&pr)[kEpt], const uint32_t (&rw)[kEpt],
                                                  uint32_t cnt, uint32_t prv, uint32_t nxt, T *__restrict__ y,
-                                                 const coo_carry<T> &cw, coo_ws_header *hdr) {
+                                                 const coo_carry<T> &cw, coo_ws_header *hdr, uint32_t row0 = 0u) {
   const uint32_t lane = threadIdx.x & 31u;
   const bool active = cnt > 0;
   const uint32_t last_lane = (c1 - g0 - 1u) / kEpt;
@@ -1136,6 +1141,13 @@ __device__ __forceinline__ void warp_tile_reduce(uint32_t wt, uint32_t g0, uint3
     if (lane >= o && (closed & (((1u << o) - 1u) << (lane + 1u - o))) == 0u) v = add_rn(a, v);
   }
   const T cin_val = __shfl_up_sync(0xffffffffu, v, 1);  // lane - 1's chain: the row rf when cont
+  if (SLICE) {
+    const uint32_t tile_last = __shfl_sync(0xffffffffu, rl, last_lane);
+    if (prv == kNoRow)
+      for (uint32_t r = lane; r < tile_first && r < n_rows; r += 32u) y[r] = T(0);
+    if (nxt == kNoRow && tile_last < n_rows)
+      for (uint32_t r = tile_last + 1u + lane; r < n_rows; r += 32u) y[r] = T(0);
+  }
   if (!active) return;
   // the lane's first run, with the carry of the lanes before it
   const T ftot = cont ? add_rn(cin_val, sf) : sf;
@@ -1146,7 +1158,7 @@ __device__ __forceinline__ void warp_tile_reduce(uint32_t wt, uint32_t g0, uint3
   // row are left to the fix-up pass, which spreads them over its grid
   if (!ACCUM) {
     if (lane == 0 && prv == kNoRow) {
-      hdr->first_row = rf;
+      if (!SLICE) hdr->first_row = rf;
     } else {
       const uint32_t lo = lane == 0 ? prv + 1u : prev_last + 1u;
       for (uint32_t r = lo; r < rf && r < n_rows; ++r) y[r] = T(0);
@@ -1167,7 +1179,7 @@ __device__ __forceinline__ void warp_tile_reduce(uint32_t wt, uint32_t g0, uint3
   } else if (lane == last_lane) {
     // the tail row continues into the next tile
     cw.tail[wt] = ltot;
-    cw.tail_row[wt] = rl;
+    cw.tail_row[wt] = rl + row0;
     if (l_from_prev) cw.head[wt] = ltot;
   }
   if (lane == last_lane) {
@@ -1176,7 +1188,7 @@ __device__ __forceinline__ void warp_tile_reduce(uint32_t wt, uint32_t g0, uint3
     if (rl == nxt) f |= kTailCont;          // its last row goes on in the next tile
     if (tile_first == rl) f |= kOneRow;
     cw.flags[wt] = f;
-    if (!ACCUM && c1 == nnz) hdr->last_row = rl;  // the fix-up pass zeroes the rows after it
+    if (!ACCUM && !SLICE && c1 == nnz) hdr->last_row = rl;  // the fix-up pass zeroes the rows after it
   }
 }
 
@@ -1729,6 +1741,110 @@ __global__ void __launch_bounds__(kBlock, sizeof(T) == 4 ? MFP_SCOO_MINBLOCKS : 
   for (uint32_t i = threadIdx.x; i < nrows; i += kBlock) y[row0 + i] = acc[i];
 }
 
+
+// ---------------------------------------------------------------------------
+// Row-ordered SCOO handles, in two passes: every slice's 256-element tiles
+// (from the slice's first element, rounded down to 8) as independent warps,
+// taken from a tile table, then a fix-up of the rows that cross tiles.  The
+// tiles, their reduction and the order of a crossing row's partial sums are
+// scoo_kernel's, so the bits are too; what changes is that a slice is no
+// longer one CTA's work.  One CTA per slice is bound by the heaviest slice: a
+// 1M-row power-law matrix (FP64, mean 7.5, rows up to 50,000) has a slice of
+// 200 tiles among slices of 15, and took 107 us there, 59 us here (the chip's
+// random x gathers are what is left).  At 8 CTAs per SM the FP32 kernel spills
+// (4M-row power-law 176 us against 170 at 6).
+// ---------------------------------------------------------------------------
+struct scoo_tile {
+  uint32_t g0;     // first element, rounded down to a multiple of 8
+  uint32_t c1;     // one past the last element
+  uint32_t slice;
+  uint32_t flags;  // bits 0-2: elements of [g0, g0 + 8) that precede the slice; below
+};
+constexpr uint32_t kSliceFirst = 8u, kSliceLast = 16u, kSliceEmpty = 32u;
+
+template <typename T, int VEC, bool R16>
+__global__ void __launch_bounds__(kBlock, sizeof(T) == 4 ? MFP_SCOO_MINBLOCKS : MFP_COO_MINBLOCKS64)
+    scoo_tile_kernel(uint32_t n_rows, uint32_t slice_size, uint32_t n_tiles, const uint4 *__restrict__ tiles,
+                     const T *__restrict__ vals, const uint32_t *__restrict__ cidx,
+                     const uint32_t *__restrict__ ridx, const uint16_t *__restrict__ rel, const T *__restrict__ x,
+                     T *__restrict__ y, coo_carry<T> cw) {
+  const uint32_t lane = threadIdx.x & 31u;
+  const uint32_t wt = blockIdx.x * (kBlock / 32u) + (threadIdx.x >> 5);
+  if (wt >= n_tiles) return;  // whole warps only
+  const uint64_t pol = policy_evict_first();
+  const uint4 tl = __ldg(tiles + wt);
+  const uint32_t g0 = tl.x, c1 = tl.y, row0 = tl.z * slice_size, flags = tl.w;
+  const uint32_t nrows = min(slice_size, n_rows - row0);
+  if (flags & kSliceEmpty) {
+    for (uint32_t r = lane; r < nrows; r += 32u) y[row0 + r] = T(0);
+    if (lane == 0) cw.flags[wt] = 0u;
+    return;
+  }
+  const uint32_t c0 = g0 + (flags & 7u);
+  T pr[kEpt];
+  uint32_t rw[kEpt], i0 = 0, cnt, prv = kNoRow, nxt = kNoRow;
+  if (R16) {  // the offsets are the slice-local rows
+    cnt = load_run_group16<T, VEC>(vals, cidx, rel, 0u, x_global<T>{x}, g0 + lane * kEpt, c0, c1, pr, rw, i0, pol);
+    if (!(flags & kSliceFirst)) prv = ld_stream_u16(rel + c0 - 1u, pol);
+    if (!(flags & kSliceLast)) nxt = ld_stream_u16(rel + c1, pol);
+  } else {
+    cnt = load_run_group<T, VEC>(vals, cidx, ridx, x_global<T>{x}, g0 + lane * kEpt, c0, c1, pr, rw, i0, pol);
+#pragma unroll
+    for (int k = 0; k < kEpt; ++k) rw[k] -= row0;
+    if (!(flags & kSliceFirst)) prv = __ldg(ridx + c0 - 1u) - row0;
+    if (!(flags & kSliceLast)) nxt = __ldg(ridx + c1) - row0;
+  }
+  warp_tile_reduce<T, false, true>(wt, g0, c1, 0u, nrows, pr, rw, cnt, prv, nxt, y + row0, cw, nullptr, row0);
+}
+
+// Pass 2: lane l of a warp owns tile 32 w + l.  A row that starts in a tile
+// and crosses into the next ones is its tail plus the following tiles' heads
+// in tile order, up to the tile where it ends.  Most end in the next tile;
+// the others are walked by the whole warp, 32 tiles' heads per round in
+// flight, the sum still one addition after the other.
+template <typename T>
+__global__ void __launch_bounds__(kBlock) scoo_fixup_kernel(uint32_t n_tiles, uint32_t n_rows, coo_carry<T> cw,
+                                                            T *__restrict__ y) {
+  griddep_wait();  // the tile pass's carries
+  const uint32_t w = blockIdx.x * kBlock + threadIdx.x, lane = threadIdx.x & 31u;
+  const uint32_t f = w < n_tiles ? cw.flags[w] : 0u;
+  const bool chain = (f & kTailCont) && !((f & kOneRow) && (f & kHeadCont));
+  T acc = T(0);
+  uint32_t row = 0;
+  bool more = false;
+  if (chain) {  // the last tile of a slice never continues, so tile w + 1 exists
+    acc = add_rn(cw.tail[w], cw.head[w + 1u]);
+    row = cw.tail_row[w];
+    const uint32_t g = cw.flags[w + 1u];
+    more = (g & kOneRow) && (g & kTailCont);
+  }
+  for (uint32_t todo = __ballot_sync(0xffffffffu, more); todo; todo &= todo - 1u) {
+    const uint32_t src = __ffs(todo) - 1u;
+    uint32_t base = __shfl_sync(0xffffffffu, w, src) + 2u;
+    T sum = __shfl_sync(0xffffffffu, acc, src);
+    uint32_t g = base + lane < n_tiles ? cw.flags[base + lane] : 0u;
+    T h = base + lane < n_tiles ? cw.head[base + lane] : T(0);
+    for (;;) {
+      // the next round's loads are in flight while this round is added up
+      const uint32_t k = base + 32u + lane;
+      const uint32_t g2 = k < n_tiles ? cw.flags[k] : 0u;
+      const T h2 = k < n_tiles ? cw.head[k] : T(0);
+      const uint32_t ends = __ballot_sync(0xffffffffu, !((g & kOneRow) && (g & kTailCont)));
+      const uint32_t n = ends ? (uint32_t)__ffs(ends) : 32u;  // heads to add, the ending tile's included
+#pragma unroll
+      for (uint32_t j = 0; j < 32; ++j) {
+        const T hj = __shfl_sync(0xffffffffu, h, j);
+        if (j < n) sum = add_rn(sum, hj);
+      }
+      if (ends) break;
+      base += 32u;
+      g = g2;
+      h = h2;
+    }
+    if (lane == src) acc = sum;
+  }
+  if (chain && row < n_rows) y[row] = acc;
+}
 
 // SCOO with the slices' elements in column order (the reference's sort_cols
 // layout, scoo_matrix_class.cpp:102-138): rows are not contiguous within a

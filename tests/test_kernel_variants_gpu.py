@@ -1,0 +1,85 @@
+"""Kernel variants chosen by a matrix's sizes and structure, at the sizes where
+they can go wrong: remainders, tile and slice edges, the ends of their ranges."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+from matrix_format_performance_b200 import formats as F  # noqa: E402
+from matrix_format_performance_b200 import synth  # noqa: E402
+from matrix_format_performance_b200._capi import call  # noqa: E402
+from matrix_format_performance_b200.device import SCOO, DeviceMatrix  # noqa: E402
+
+TOL = {np.float32: 1e-5, np.float64: 1e-12}  # per row, of sum |a_ij x_j|
+
+
+def dev(a):
+    return torch.from_numpy(np.ascontiguousarray(a)).cuda()
+
+
+def p(t):
+    return C.c_void_p(t.data_ptr())
+
+
+def check(oracle_lib, m, x, y, what):
+    ys, ab = oracle_lib.csr_spmv_exact(m.rows, m.row_ptr, m.columns, m.data, x)
+    bad = ~(np.abs(y.astype(np.float64) - ys) <= TOL[m.dtype.type] * ab)
+    assert not bad.any(), f"{what}: {int(bad.sum())} rows, first {int(np.argmax(bad))}"
+
+
+def csr(lens, cols, dtype, seed=3):
+    """Random columns (repeats allowed), values U[-1, 1]."""
+    rng = np.random.default_rng(seed)
+    rp = np.zeros(len(lens) + 1, np.int64)
+    rp[1:] = np.cumsum(lens)
+    row = np.repeat(np.arange(len(lens)), lens)
+    c = rng.integers(0, cols, int(rp[-1]))
+    c = c[np.lexsort((c, row))].astype(np.uint32)
+    return F.csr_matrix_class.from_arrays(len(lens), cols, rp.astype(np.uint32), c, rng.uniform(-1, 1, len(c)), dtype)
+
+
+def spmv(dm, m, x):
+    xt, y = dev(x), torch.full((m.rows,), float("nan"), dtype=dev(x).dtype, device="cuda")
+    dm.spmv(xt, y)
+    torch.cuda.synchronize()
+    return y.cpu().numpy()
+
+
+def uneven_lengths(case):
+    rng = np.random.default_rng(8)
+    lens = rng.integers(0, 13, 3000)
+    if case == "long_rows":     # crossing chains of 250, 36 and 2 tiles, one of them ending a slice
+        lens[700], lens[1500], lens[2099] = 64_000, 9_001, 400
+    elif case == "holes":       # empty slices (21 rows each) at the start, inside and at the end
+        lens[:63], lens[1008:1050], lens[2900:] = 0, 0, 0
+        lens[1700] = 20_011
+    else:                       # one row holds almost everything
+        lens[:] = 0
+        lens[[5, 2999]] = 50_003, 1
+    return lens
+
+
+@pytest.mark.parametrize("case", ["long_rows", "holes", "one_row"])
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+def test_scoo_tiles_give_the_bits_of_one_cta_per_slice(oracle_lib, case, dtype):
+    """Uneven SCOO slices run as independent warp tiles; the raw entry point
+    keeps one CTA per slice.  Same tiles, same order of a crossing row's
+    partial sums: the same bits."""
+    m = csr(uneven_lengths(case), 5_000, dtype)
+    x = synth.vector(4, m.cols).astype(dtype)
+    s = F.scoo_matrix_class(148, 49152, m)
+    dm = DeviceMatrix.build(m, SCOO)
+    assert dm.info().kernel_launches == 2  # tiles and fix-up
+    y = spmv(dm, m, x)
+    dm.close()
+    keep = [dev(a) for a in (s.values, s.c_index.view(np.int32), s.r_index.view(np.int32), s.slices_ptr.view(np.int32), x)]
+    raw = torch.full((m.rows,), float("nan"), dtype=keep[0].dtype, device="cuda")
+    v, ci, ri, sp, xt = (p(t) for t in keep)
+    call(f"mfp_scoo_spmv_{'f32' if dtype == np.float32 else 'f64'}", m.rows, m.cols, s.slices_count, s.slice_size, v, ci,
+         ri, sp, None, 0, None, xt, p(raw), None)
+    torch.cuda.synchronize()
+    check(oracle_lib, m, x, y, case)
+    assert np.array_equal(raw.cpu().numpy().view(np.uint8), y.view(np.uint8))
