@@ -83,3 +83,26 @@ def test_scoo_tiles_give_the_bits_of_one_cta_per_slice(oracle_lib, case, dtype):
     torch.cuda.synchronize()
     check(oracle_lib, m, x, y, case)
     assert np.array_equal(raw.cpu().numpy().view(np.uint8), y.view(np.uint8))
+
+
+def test_scoo_tiles_on_two_streams_and_in_a_graph():
+    """One handle used from two streams at once and from a captured graph:
+    each call has its own carries."""
+    m = csr(uneven_lengths("long_rows"), 5_000, np.float32)
+    dm = DeviceMatrix.build(m, SCOO)
+    xs = [dev(synth.vector(k, m.cols).astype(np.float32)) for k in range(3)]
+    want = [spmv(dm, m, x.cpu().numpy()) for x in xs]
+    ys = [torch.zeros(m.rows, device="cuda") for _ in xs]
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        dm.spmv(xs[2], ys[2])
+    for _ in range(20):
+        for s, x, y in zip(streams, xs, ys):
+            dm.spmv(x, y, s)
+        graph.replay()
+    torch.cuda.synchronize()
+    del graph
+    dm.close()
+    for w, y in zip(want, ys):
+        assert np.array_equal(w.view(np.uint32), y.cpu().numpy().view(np.uint32))
