@@ -162,8 +162,16 @@ def check(status: int) -> None:
         raise MfpError(status, msg.decode() if msg else "")
 
 
+_bound: dict = {}  # name -> bound function: an attribute lookup on the CDLL costs as much as a small call
+
+
 def call(name: str, *args) -> None:
-    check(getattr(load(), name)(*args))
+    fn = _bound.get(name)
+    if fn is None:
+        fn = _bound[name] = getattr(load(), name)
+    status = fn(*args)
+    if status:
+        check(status)
 
 
 class BatchConfig(C.Structure):

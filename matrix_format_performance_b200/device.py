@@ -38,19 +38,37 @@ def _cfg(config: dict | None):
     return C.byref(c)
 
 
-def _dptr(t) -> C.c_void_p:
-    """Device pointer of a torch tensor (or an int address)."""
+# The host path of a small product: plain int addresses (ctypes converts them
+# to void* by the declared argument types) and the current stream's raw handle
+# without a torch Stream object.  A 128 x 128 Laplacian's product, back to back,
+# went from 9.2 to 6.2 us a call (ELL 8.0 -> 4.1).
+def _dptr(t) -> int:
+    """Device address of a torch tensor (or an int address)."""
     if isinstance(t, int):
-        return C.c_void_p(t)
+        return t
     assert t.is_cuda and t.is_contiguous()
-    return C.c_void_p(t.data_ptr())
+    return t.data_ptr()
 
 
-def _stream(stream) -> C.c_void_p:
+_current = None  # () -> the current stream's handle
+
+
+def _bind_current():
+    import torch
+    torch.cuda.current_stream()  # initialises CUDA, or raises
+    raw, device = getattr(torch._C, "_cuda_getCurrentRawStream", None), getattr(torch._C, "_cuda_getDevice", None)
+    if raw is None or device is None:
+        return lambda: torch.cuda.current_stream().cuda_stream
+    return lambda: raw(device())
+
+
+def _stream(stream) -> int:
     if stream is None:
-        import torch
-        stream = torch.cuda.current_stream()
-    return C.c_void_p(int(getattr(stream, "cuda_stream", stream)))
+        global _current
+        if _current is None:
+            _current = _bind_current()
+        return _current()
+    return int(getattr(stream, "cuda_stream", stream))
 
 
 class DeviceMatrix:
