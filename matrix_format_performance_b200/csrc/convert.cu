@@ -10,9 +10,9 @@
 //     the first position of every row that starts inside it with the row id,
 //     then an inclusive max-scan over the tile gives each position its row
 //     (empty rows never mark a position, long rows span tiles);
-//   - a stable LSD radix sort (8-bit digits, per-tile histograms in
-//     digit-major order, stable in-tile ranking by warp match) for COO
-//     triplets -> CSR on the composite key (row, column).
+//   - a stable LSD radix sort (digits of up to 9 bits, one launch per digit:
+//     tiles rank their keys, look back for the counts of the tiles before them
+//     and scatter) for COO triplets -> CSR on the composite key (row, column).
 #include "host_common.h"
 
 #include <cuda_runtime.h>
@@ -31,8 +31,15 @@ constexpr uint32_t kThreads = 256;
 constexpr uint32_t kWarps = kThreads / 32;
 constexpr uint32_t kItems = 8;
 constexpr uint32_t kTile = kThreads * kItems;  // items per CTA in scans and expansions
-constexpr uint32_t kRadixRounds = 16;
-constexpr uint32_t kRadixTile = kThreads * kRadixRounds;  // keys per CTA in a radix pass
+constexpr uint32_t kRadixThreads = 512;
+constexpr uint32_t kRadixWarps = kRadixThreads / 32;
+constexpr uint32_t kRadixRounds = 12;
+constexpr uint32_t kRadixTile = kRadixThreads * kRadixRounds;  // keys per CTA in a radix pass
+constexpr uint32_t kRadixBits = 9;                             // widest digit
+constexpr uint32_t kRadixBins = 1u << kRadixBits;
+static_assert(kRadixBins == kRadixThreads, "one thread per digit");
+constexpr uint32_t kRadixPasses = 8;                      // 64-bit keys
+constexpr uint32_t kRadixPolls = 1u << 20;                // look-back limit, about a second
 
 int cuda_fail(cudaError_t e, const char *what) {
   return fail(MFP_ERROR_CUDA, "%s: %s", what, cudaGetErrorString(e));
@@ -96,10 +103,6 @@ __device__ __forceinline__ uint32_t block_excl(uint32_t v, uint32_t *s, uint32_t
 // ---------------------------------------------------------------------------
 // Exclusive scan of f(i), i in [0, n): out[0..n], out[n] = the total.
 // ---------------------------------------------------------------------------
-struct f_counts {
-  const uint32_t *c;
-  __device__ uint32_t operator()(uint32_t i) const { return c[i]; }
-};
 // in-row positions >= start of row i (coo_matrix_class tail, matrix_converter.cpp:242-257)
 struct f_tail {
   const uint32_t *rp;
@@ -523,149 +526,298 @@ __global__ void __launch_bounds__(kThreads) scoo_windows_kernel(uint32_t nnz, co
 // ---------------------------------------------------------------------------
 // COO triplets -> CSR: keys (row << cb | col) with the value converted to T as
 // payload, a stable LSD radix sort when the input is not already in CSR
-// order, then row_ptr from the row boundaries of the sorted keys.
+// order, then row_ptr from the row boundaries of the sorted rows.
+//
+// One launch per digit.  A pass reads and writes 12 bytes per FP32 element (24
+// in all); the histograms of every digit come from one read of the ids before
+// the passes, the first pass reads the triplets themselves and the last one
+// writes the CSR arrays.  B200, 15.1M elements of 2M rows (42 key bits), FP32:
+// 920 us: 74 for the histograms and 150 a pass (2.4 TB/s; shared memory at 56%
+// and instruction issue at 50% of their rates, 32 warps per SM).  It was 1,340
+// us with five launches per 8-bit digit (histogram 39 us, scans 12, scatter
+// 137, whose __match_any_sync kept one pipe 74% busy), 130 for making the keys
+// and 100 for splitting them.  Equal digits found with a shared-memory atomicOr
+// instead of ballots: 988 us; 256 threads with 16 keys each: 1,259 us (spills,
+// runs of 8 keys).
 // ---------------------------------------------------------------------------
-constexpr uint32_t kKeyBlocks = 148 * 8;
+constexpr uint32_t kKeyBlocks = 148 * 6;
 
-// err[0] |= 1 (row id) / 2 (col id), err[1] = first bad element; err[2] = 1
-// when some key is smaller than its predecessor (input not in CSR order)
-template <typename T>
-__global__ void __launch_bounds__(kThreads) make_keys_kernel(uint32_t nnz, uint32_t rows, uint32_t cols,
-                                                             const uint32_t *__restrict__ ri,
-                                                             const uint32_t *__restrict__ ci,
-                                                             const double *__restrict__ v, uint32_t cb,
-                                                             unsigned long long *__restrict__ keys,
-                                                             T *__restrict__ pay, uint32_t *err) {
-  bool unsorted = false;
-  for (uint64_t i = (uint64_t)blockIdx.x * kThreads + threadIdx.x; i < nnz; i += (uint64_t)gridDim.x * kThreads) {
-    const uint32_t r = ri[i], c = ci[i];
-    if (r >= rows || c >= cols) {
-      atomicOr(&err[0], r >= rows ? 1u : 2u);
-      atomicMin(&err[1], (uint32_t)i);
-    }
-    const unsigned long long k = ((unsigned long long)r << cb) | c;
-    keys[i] = k;
-    pay[i] = static_cast<T>(v[i]);
-    if (i && (((unsigned long long)ri[i - 1] << cb) | ci[i - 1]) > k) unsorted = true;
+struct radix_digits {
+  uint32_t passes = 0, bits = 0;  // digits per key, bits per digit
+  radix_digits() = default;
+  explicit radix_digits(uint32_t key_bits) {
+    passes = (key_bits + kRadixBits - 1u) / kRadixBits;
+    bits = key_bits <= 8u * passes ? 8u : 9u;
   }
-  if (__syncthreads_or(unsorted) && threadIdx.x == 0) err[2] = 1u;
-}
-
-__global__ void __launch_bounds__(kThreads) radix_hist_kernel(uint32_t n, const unsigned long long *keys,
-                                                              uint32_t shift, uint32_t tiles, uint32_t *counts) {
-  __shared__ uint32_t h[256];
-  h[threadIdx.x] = 0u;
-  __syncthreads();
-  const uint64_t base = (uint64_t)blockIdx.x * kRadixTile;
-#pragma unroll 4
-  for (uint32_t j = 0; j < kRadixRounds; ++j) {
-    const uint64_t i = base + j * kThreads + threadIdx.x;
-    if (i < n) atomicAdd(&h[(uint32_t)(keys[i] >> shift) & 255u], 1u);
-  }
-  __syncthreads();
-  counts[(size_t)threadIdx.x * tiles + blockIdx.x] = h[threadIdx.x];
-}
-
-// Stable scatter of one 4096-key tile: keys go, in tile order, after every key
-// of a smaller digit and after the same digit's keys of earlier tiles
-// (offsets = exclusive scan of the digit-major tile histograms).  Warp w ranks
-// its contiguous 512 keys with a warp-private digit histogram (warp match for
-// equal digits), the warps' counts are scanned per digit, the tile is placed
-// in shared memory in digit order and written out as contiguous digit runs.
-template <typename P>
-struct radix_smem {
-  unsigned long long key[kRadixTile];
-  P pay[kRadixTile];
-  uint32_t wh[kWarps][256];
-  uint32_t gbase[256], start[256];
-  uint32_t red[kWarps];
 };
 
+// Where a pass takes its keys and payloads, and where it puts them.
+template <typename T>
+struct triplets_in {
+  const uint32_t *__restrict__ r, *__restrict__ c;
+  const double *__restrict__ v;
+  uint32_t cb;
+  __device__ unsigned long long key(uint64_t i) const { return ((unsigned long long)r[i] << cb) | c[i]; }
+  __device__ T pay(uint64_t i) const { return static_cast<T>(v[i]); }
+};
 template <typename P>
-__global__ void __launch_bounds__(kThreads) radix_scatter_kernel(uint32_t n, const unsigned long long *keys,
-                                                                 const P *pay, uint32_t shift, uint32_t tiles,
-                                                                 const uint32_t *offsets,
-                                                                 unsigned long long *keys_out, P *pay_out) {
+struct pairs_in {
+  const unsigned long long *__restrict__ k;
+  const P *__restrict__ p;
+  __device__ unsigned long long key(uint64_t i) const { return k[i]; }
+  __device__ P pay(uint64_t i) const { return p[i]; }
+};
+template <typename P>
+struct pairs_out {
+  unsigned long long *__restrict__ k;
+  P *__restrict__ p;
+  __device__ void key(uint32_t g, unsigned long long v) const { k[g] = v; }
+  __device__ void pay(uint32_t g, P v) const { p[g] = v; }
+};
+template <typename T>
+struct csr_out {
+  uint32_t *__restrict__ rows, *__restrict__ cols;
+  T *__restrict__ data;
+  uint32_t cb;
+  __device__ void key(uint32_t g, unsigned long long v) const {
+    rows[g] = (uint32_t)(v >> cb);
+    cols[g] = (uint32_t)(v & ((1ull << cb) - 1ull));
+  }
+  __device__ void pay(uint32_t g, T v) const { data[g] = v; }
+};
+
+template <uint32_t BITS>
+__device__ __forceinline__ uint32_t digit_of(unsigned long long k, uint32_t shift) {
+  const uint32_t lo = (uint32_t)k, hi = (uint32_t)(k >> 32);
+  return (shift < 32u ? __funnelshift_r(lo, hi, shift) : hi >> (shift - 32u)) & ((1u << BITS) - 1u);
+}
+
+// Exclusive prefix over the CTA of a radix pass; s holds kRadixWarps words.
+__device__ __forceinline__ uint32_t radix_excl(uint32_t v, uint32_t *s) {
+  const uint32_t lane = threadIdx.x & 31u, w = threadIdx.x >> 5;
+  const uint32_t inc = warp_incl_sum(v);
+  if (lane == 31) s[w] = inc;
+  __syncthreads();
+  if (w == 0) {
+    const uint32_t t = warp_incl_sum(lane < kRadixWarps ? s[lane] : 0u);
+    if (lane < kRadixWarps) s[lane] = t;
+  }
+  __syncthreads();
+  return (w ? s[w - 1] : 0u) + inc - v;
+}
+
+// Histograms of every digit: hist[pass][bin] (zeroed).  CHECK (triplets): err[0]
+// |= 1 (row id) / 2 (col id), err[1] = first bad element, err[2] = 1 when some
+// key is smaller than its predecessor (input not in CSR order).
+template <bool CHECK, uint32_t BITS, typename In>
+__global__ void __launch_bounds__(kThreads) radix_hist_kernel(uint32_t n, In in, uint32_t rows, uint32_t cols,
+                                                              uint32_t passes, uint32_t *hist, uint32_t *err) {
+  __shared__ uint32_t h[kRadixPasses * kRadixBins];
+  for (uint32_t i = threadIdx.x; i < passes * kRadixBins; i += kThreads) h[i] = 0u;
+  __syncthreads();
+  bool unsorted = false;
+  // tiles of 4 keys per thread, their loads issued together
+  const uint64_t step = (uint64_t)gridDim.x * kThreads * 4u;
+  for (uint64_t b = (uint64_t)blockIdx.x * kThreads * 4u; b < n; b += step) {
+    unsigned long long k[4];
+    bool bad[4];
+#pragma unroll
+    for (uint32_t j = 0; j < 4; ++j) {
+      const uint64_t i = b + j * kThreads + threadIdx.x;
+      bad[j] = false;
+      if constexpr (CHECK) {
+        const uint32_t r = i < n ? in.r[i] : 0u, c = i < n ? in.c[i] : 0u;
+        k[j] = ((unsigned long long)r << in.cb) | c;
+        bad[j] = i < n && (r >= rows || c >= cols);
+      } else {
+        k[j] = i < n ? in.key(i) : 0ull;
+      }
+    }
+#pragma unroll
+    for (uint32_t j = 0; j < 4; ++j) {
+      const uint64_t i = b + j * kThreads + threadIdx.x;
+      if constexpr (CHECK) {
+        unsigned long long prev = __shfl_up_sync(0xffffffffu, k[j], 1);
+        if ((threadIdx.x & 31u) == 0) prev = i && i < n ? in.key(i - 1) : 0ull;
+        unsorted |= i < n && prev > k[j];
+        if (bad[j]) {
+          atomicOr(&err[0], in.r[i] >= rows ? 1u : 2u);
+          atomicMin(&err[1], (uint32_t)i);
+        }
+      }
+      if (i < n) {
+#pragma unroll
+        for (uint32_t p = 0; p < kRadixPasses; ++p)
+          if (p < passes) atomicAdd(&h[p * kRadixBins + digit_of<BITS>(k[j], p * BITS)], 1u);
+      }
+    }
+  }
+  if (CHECK && unsorted) err[2] = 1u;
+  __syncthreads();
+  for (uint32_t i = threadIdx.x; i < passes * kRadixBins; i += kThreads)
+    if (h[i]) atomicAdd(&hist[i], h[i]);
+}
+
+// Status words of the look-back, one per (tile, digit): the high half says
+// what the low half counts, by pass (stale words of earlier passes say less).
+__device__ __forceinline__ unsigned long long status_word(uint32_t pass, bool prefix, uint32_t v) {
+  return ((unsigned long long)(2u * pass + (prefix ? 2u : 1u)) << 32) | v;
+}
+__device__ __forceinline__ unsigned long long ld_status(const unsigned long long *p) {
+  unsigned long long v;
+  asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ void st_status(unsigned long long *p, unsigned long long v) {
+  asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
+
+// One digit: stable scatter of a 6,144-key tile.  Keys go, in tile order, after
+// every key of a smaller digit and after the same digit's keys of earlier
+// tiles.  Warp w ranks its contiguous 384 keys with a warp-private digit
+// histogram (equal digits found bit by bit with ballots), thread t scans digit
+// t over the warps and looks back for its count in the tiles before, the tile
+// is placed in shared memory in digit order and written out as contiguous digit
+// runs; payloads follow through the same shared memory.  Tiles are numbered in
+// the order their CTAs start, so a tile only ever waits for CTAs that are
+// running; the wait is bounded (err[3]).
+struct radix_smem {
+  unsigned long long key[kRadixTile];  // or payloads
+  uint32_t wh[kRadixWarps][kRadixBins];
+  uint32_t gbase[kRadixBins];
+  uint32_t red[kRadixWarps], red2[kRadixWarps];
+  uint32_t tile;
+};
+template <uint32_t BITS, typename P, typename In, typename Out>
+__global__ void __launch_bounds__(kRadixThreads, 2) radix_pass_kernel(uint32_t n, In in, Out out, uint32_t pass,
+                                                                      const uint32_t *hist, uint32_t *counter,
+                                                                      unsigned long long *status, uint32_t *err) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  radix_smem<P> &S = *reinterpret_cast<radix_smem<P> *>(smem_raw);
-  constexpr uint32_t kPerWarp = kRadixTile / kWarps;
+  radix_smem &S = *reinterpret_cast<radix_smem *>(smem_raw);
+  constexpr uint32_t kPerWarp = kRadixTile / kRadixWarps;
   const uint32_t t = threadIdx.x, lane = t & 31u, warp = t >> 5;
-  const uint64_t base = (uint64_t)blockIdx.x * kRadixTile;
+  if (t == 0) S.tile = atomicAdd(counter, 1u);
+#pragma unroll
+  for (uint32_t i = 0; i < kRadixWarps; ++i) S.wh[i][t] = 0u;
+  const uint32_t hv = hist[t];
+  __syncthreads();
+  const uint32_t tile = S.tile, shift = pass * BITS;
+  const uint64_t base = (uint64_t)tile * kRadixTile;
   const uint32_t tn = (uint32_t)min((uint64_t)kRadixTile, n - base);
-  const uint32_t wbase = warp * kPerWarp;
+  const uint32_t wbase = warp * kPerWarp + lane;
   unsigned long long k[kRadixRounds];
-  P v[kRadixRounds];
 #pragma unroll
-  for (uint32_t j = 0; j < kRadixRounds; ++j) {
-    const uint32_t p = wbase + j * 32u + lane;
-    k[j] = p < tn ? keys[base + p] : 0ull;
-    v[j] = p < tn ? pay[base + p] : P(0);
-  }
-#pragma unroll
-  for (uint32_t w = 0; w < kWarps; ++w) S.wh[w][t] = 0u;
-  S.gbase[t] = offsets[(size_t)t * tiles + blockIdx.x];
-  __syncthreads();
+  for (uint32_t j = 0; j < kRadixRounds; ++j) k[j] = wbase + j * 32u < tn ? in.key(base + wbase + j * 32u) : ~0ull;
+  // the keys of smaller digits in the whole array
+  const uint32_t below = radix_excl(hv, S.red);
   uint32_t rk[kRadixRounds];
+  uint32_t *wh = S.wh[warp];
 #pragma unroll
   for (uint32_t j = 0; j < kRadixRounds; ++j) {
-    const bool valid = wbase + j * 32u + lane < tn;
-    const uint32_t d = valid ? (uint32_t)(k[j] >> shift) & 255u : 256u;  // 256: never a digit
-    const uint32_t peers = __match_any_sync(0xffffffffu, d);
-    const uint32_t before = valid ? S.wh[warp][d] : 0u;
+    const uint32_t d = digit_of<BITS>(k[j], shift);
+    const bool valid = wbase + j * 32u < tn;
+    uint32_t peers = __ballot_sync(0xffffffffu, valid);
+#pragma unroll
+    for (uint32_t b = 0; b < BITS; ++b) {
+      const uint32_t other = 0u - ((d >> b) & 1u ^ 1u);  // all ones where the bit is 0
+      peers &= __ballot_sync(0xffffffffu, (d >> b) & 1u) ^ other;
+    }
+    const uint32_t before = wh[d];
     __syncwarp();
-    if (valid && lane == (uint32_t)(__ffs(peers) - 1)) S.wh[warp][d] = before + __popc(peers);
+    const uint32_t mine = peers & ((1u << lane) - 1u);
+    if (valid && mine == 0u) wh[d] = before + __popc(peers);
     __syncwarp();
-    rk[j] = before + __popc(peers & ((1u << lane) - 1u));
+    rk[j] = before + __popc(mine);
   }
   __syncthreads();
-  uint32_t tot = 0;  // thread t: digit t
+  uint32_t tot = 0;  // thread t: digit t, summed over the warps
 #pragma unroll
-  for (uint32_t w = 0; w < kWarps; ++w) {
-    const uint32_t c = S.wh[w][t];
-    S.wh[w][t] = tot;
-    tot += c;
-  }
-  S.start[t] = block_excl<false>(tot, S.red, nullptr);
-  __syncthreads();
+  for (uint32_t w = 0; w < kRadixWarps; ++w) tot += S.wh[w][t];
+  unsigned long long *mine = status + (size_t)tile * kRadixBins + t;
+  st_status(mine, status_word(pass, tile == 0, tot));
+  const uint32_t start = radix_excl(tot, S.red2);
+  {
+    uint32_t at = start;
 #pragma unroll
-  for (uint32_t j = 0; j < kRadixRounds; ++j) {
-    if (wbase + j * 32u + lane < tn) {
-      const uint32_t d = (uint32_t)(k[j] >> shift) & 255u;
-      const uint32_t lp = S.start[d] + S.wh[warp][d] + rk[j];
-      S.key[lp] = k[j];
-      S.pay[lp] = v[j];
+    for (uint32_t w = 0; w < kRadixWarps; ++w) {
+      const uint32_t c = S.wh[w][t];
+      S.wh[w][t] = at;
+      at += c;
     }
   }
   __syncthreads();
-  for (uint32_t p = t; p < tn; p += kThreads) {
-    const unsigned long long kk = S.key[p];
-    const uint32_t d = (uint32_t)(kk >> shift) & 255u;
-    const uint32_t g = S.gbase[d] + (p - S.start[d]);
-    keys_out[g] = kk;
-    pay_out[g] = S.pay[p];
+#pragma unroll
+  for (uint32_t j = 0; j < kRadixRounds; ++j)
+    if (wbase + j * 32u < tn) {
+      rk[j] += wh[digit_of<BITS>(k[j], shift)];  // the key's place in the tile
+      S.key[rk[j]] = k[j];
+    }
+  // the same digit's keys in earlier tiles
+  uint32_t excl = 0;
+  if (tile) {
+    const unsigned long long *st = status + t;
+    for (uint32_t w = tile - 1u, polls = 0;;) {
+      const unsigned long long v = ld_status(st + (size_t)w * kRadixBins);
+      const uint32_t flag = (uint32_t)(v >> 32);
+      if (flag <= 2u * pass) {  // not there yet
+        if (++polls > kRadixPolls) {
+          atomicOr(&err[3], 1u);
+          break;
+        }
+        continue;
+      }
+      excl += (uint32_t)v;
+      if (flag == 2u * pass + 2u || w == 0) break;
+      --w;
+    }
+    st_status(mine, status_word(pass, true, excl + tot));
   }
+  S.gbase[t] = below + excl - start;
+  __syncthreads();
+  uint32_t g[kRadixRounds];
+#pragma unroll
+  for (uint32_t j = 0; j < kRadixRounds; ++j) {
+    const uint32_t p = j * kRadixThreads + t;
+    if (p < tn) {
+      const unsigned long long kk = S.key[p];
+      g[j] = S.gbase[digit_of<BITS>(kk, shift)] + p;
+      out.key(g[j], kk);
+    }
+  }
+  P v[kRadixRounds];
+#pragma unroll
+  for (uint32_t j = 0; j < kRadixRounds; ++j)
+    v[j] = wbase + j * 32u < tn ? in.pay(base + wbase + j * 32u) : P(0);
+  __syncthreads();
+  P *sp = reinterpret_cast<P *>(S.key);
+#pragma unroll
+  for (uint32_t j = 0; j < kRadixRounds; ++j)
+    if (wbase + j * 32u < tn) sp[rk[j]] = v[j];
+  __syncthreads();
+#pragma unroll
+  for (uint32_t j = 0; j < kRadixRounds; ++j)
+    if (j * kRadixThreads + t < tn) out.pay(g[j], sp[j * kRadixThreads + t]);
 }
 
-// row_ptr from sorted keys: position p starts the rows (row(p-1), row(p)]
+// row_ptr from sorted rows: position p starts the rows (rows[p-1], rows[p]]
 // (p = nnz closes the rows after the last element's row).
-__global__ void __launch_bounds__(kThreads) rowptr_from_keys_kernel(uint32_t nnz, uint32_t rows,
-                                                                    const unsigned long long *keys, uint32_t cb,
-                                                                    uint32_t *rp) {
+__global__ void __launch_bounds__(kThreads) rowptr_from_rows_kernel(uint32_t nnz, uint32_t rows,
+                                                                    const uint32_t *__restrict__ ri, uint32_t *rp) {
   const uint64_t p = (uint64_t)blockIdx.x * kThreads + threadIdx.x;
   if (p > nnz) return;
-  const int64_t cur = p < nnz ? (int64_t)(keys[p] >> cb) : (int64_t)rows;
-  const int64_t prev = p ? (int64_t)(keys[p - 1] >> cb) : -1;
-  for (int64_t q = prev + 1; q <= cur; ++q) rp[q] = (uint32_t)p;
+  const uint32_t cur = p < nnz ? ri[p] : rows;
+  for (uint32_t q = p ? ri[p - 1] + 1u : 0u; q <= cur; ++q) rp[q] = (uint32_t)p;
 }
 
+// Triplets already in CSR order.
 template <typename T>
-__global__ void __launch_bounds__(kThreads) csr_split_kernel(uint32_t nnz, const unsigned long long *__restrict__ keys,
-                                                             const T *__restrict__ pay, unsigned long long cmask,
-                                                             uint32_t *__restrict__ cols_out, T *__restrict__ data_out) {
+__global__ void __launch_bounds__(kThreads) csr_copy_kernel(uint32_t nnz, const uint32_t *__restrict__ ci,
+                                                            const double *__restrict__ v, uint32_t *__restrict__ cols_out,
+                                                            T *__restrict__ data_out) {
   const uint32_t p = blockIdx.x * kThreads + threadIdx.x;
   if (p >= nnz) return;
-  cols_out[p] = (uint32_t)(keys[p] & cmask);
-  data_out[p] = pay[p];
+  cols_out[p] = ci[p];
+  data_out[p] = static_cast<T>(v[p]);
 }
 
 bool valid_vt(int vt) { return vt == MFP_F32 || vt == MFP_F64; }
@@ -704,32 +856,66 @@ int coo_from_csr_t(uint32_t rows, const uint32_t *rp, const uint32_t *ci, const 
   return ok();
 }
 
+// Device words of one sort: histograms, tile counters and status words, zeroed
+// by begin().
+struct radix_state {
+  uint32_t *hist = nullptr, *counters = nullptr;
+  unsigned long long *status = nullptr;
+  uint32_t tiles = 0;
+  int begin(uint32_t n, const radix_digits &dg, scratch &sc) {
+    tiles = blocks_for(n, kRadixTile);
+    const size_t words = (size_t)tiles * kRadixBins;
+    const size_t bytes = words * 8u + kRadixPasses * (kRadixBins + 1u) * 4u;
+    unsigned char *p = nullptr;
+    const int s = sc.get(&p, bytes);
+    if (s) return s;
+    status = reinterpret_cast<unsigned long long *>(p);
+    hist = reinterpret_cast<uint32_t *>(p + words * 8u);
+    counters = hist + kRadixPasses * kRadixBins;
+    CV_TRY(cudaMemsetAsync(p, 0, bytes, sc.st), "cudaMemsetAsync");
+    return MFP_SUCCESS;
+  }
+};
+template <typename P, typename In, typename Out>
+int radix_pass(uint32_t n, const In &in, const Out &out, const radix_digits &dg, uint32_t pass, const radix_state &R,
+               uint32_t *err, scratch &sc) {
+  auto k = dg.bits == 8u ? radix_pass_kernel<8, P, In, Out> : radix_pass_kernel<9, P, In, Out>;
+  CV_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(radix_smem)),
+         "cudaFuncSetAttribute");
+  k<<<R.tiles, kRadixThreads, sizeof(radix_smem), sc.st>>>(n, in, out, pass, R.hist + pass * kRadixBins,
+                                                           R.counters + pass, R.status, err);
+  CV_TRY(cudaGetLastError(), "radix_pass_kernel");
+  return MFP_SUCCESS;
+}
+int radix_error(uint32_t flag) {
+  return flag ? fail(MFP_ERROR_DEVICE_WAIT, "a radix tile gave up waiting for the tiles before it") : MFP_SUCCESS;
+}
+
 // Stable LSD radix sort of n (key, payload) pairs on the low `bits` key bits;
 // k0 / p0 hold the input and, on return, the sorted pairs (buffers swap).
 template <typename P>
 int radix_sort_pairs(uint32_t n, uint32_t bits, unsigned long long *&k0, P *&p0, scratch &sc) {
   if (n == 0 || bits == 0) return MFP_SUCCESS;
-  const uint32_t tiles = blocks_for(n, kRadixTile);
-  const uint64_t ncount = 256ull * tiles;
-  if (ncount > 0xffffffffull) return fail(MFP_ERROR_TOO_LARGE, "too many radix tiles");
+  const radix_digits dg(bits);
   unsigned long long *k1 = nullptr;
   P *p1 = nullptr;
-  uint32_t *hist = nullptr, *hoff = nullptr;
+  uint32_t *err = nullptr, h_err[4];
+  radix_state R;
   int s;
-  if ((s = sc.get(&k1, n)) || (s = sc.get(&p1, n)) || (s = sc.get(&hist, ncount)) || (s = sc.get(&hoff, ncount + 1)))
-    return s;
-  const size_t smem = sizeof(radix_smem<P>);
-  CV_TRY(cudaFuncSetAttribute(radix_scatter_kernel<P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
-         "cudaFuncSetAttribute");
-  for (uint32_t shift = 0; shift < bits; shift += 8) {
-    radix_hist_kernel<<<tiles, kThreads, 0, sc.st>>>(n, k0, shift, tiles, hist);
-    if ((s = exclusive_scan((uint32_t)ncount, f_counts{hist}, hoff, sc))) return s;
-    radix_scatter_kernel<P><<<tiles, kThreads, smem, sc.st>>>(n, k0, p0, shift, tiles, hoff, k1, p1);
-    CV_TRY(cudaGetLastError(), "radix pass");
+  if ((s = sc.get(&k1, n)) || (s = sc.get(&p1, n)) || (s = sc.get(&err, 4)) || (s = R.begin(n, dg, sc))) return s;
+  CV_TRY(cudaMemsetAsync(err, 0, 16, sc.st), "cudaMemsetAsync");
+  auto hk = dg.bits == 8u ? radix_hist_kernel<false, 8, pairs_in<P>> : radix_hist_kernel<false, 9, pairs_in<P>>;
+  hk<<<std::min(kKeyBlocks, blocks_for(n, 4u * kThreads)), kThreads, 0, sc.st>>>(n, pairs_in<P>{k0, p0}, 0u, 0u,
+                                                                                 dg.passes, R.hist, err);
+  CV_TRY(cudaGetLastError(), "radix_hist_kernel");
+  for (uint32_t pass = 0; pass < dg.passes; ++pass) {
+    if ((s = radix_pass<P>(n, pairs_in<P>{k0, p0}, pairs_out<P>{k1, p1}, dg, pass, R, err, sc))) return s;
     std::swap(k0, k1);
     std::swap(p0, p1);
   }
-  return MFP_SUCCESS;
+  CV_TRY(cudaMemcpyAsync(h_err, err, sizeof(h_err), cudaMemcpyDeviceToHost, sc.st), "cudaMemcpyAsync");
+  CV_TRY(cudaStreamSynchronize(sc.st), "cudaStreamSynchronize");
+  return radix_error(h_err[3]);
 }
 
 template <typename T>
@@ -745,27 +931,54 @@ int csr_from_coo_t(uint32_t rows, uint32_t cols, uint32_t nnz, const uint32_t *r
     return ok();
   }
   const uint32_t rb = rows > 1 ? bits_for(rows - 1) : 0u, cb = cols > 1 ? bits_for(cols - 1) : 0u;
+  const radix_digits dg(rb + cb);
   uint32_t *err = nullptr;
-  unsigned long long *k0 = nullptr;
-  T *p0 = nullptr;
+  radix_state R;
   int s;
-  if ((s = sc.get(&err, 4)) || (s = sc.get(&k0, nnz)) || (s = sc.get(&p0, nnz))) return s;
+  if ((s = sc.get(&err, 4)) || (s = R.begin(nnz, dg, sc))) return s;
   const uint32_t err_init[4] = {0u, 0xffffffffu, 0u, 0u};
   CV_TRY(cudaMemcpyAsync(err, err_init, sizeof(err_init), cudaMemcpyHostToDevice, st), "cudaMemcpyAsync");
-  make_keys_kernel<T><<<std::min(kKeyBlocks, blocks_for(nnz, kThreads)), kThreads, 0, st>>>(nnz, rows, cols, ri, ci,
-                                                                                           v, cb, k0, p0, err);
-  CV_TRY(cudaGetLastError(), "make_keys_kernel");
+  const triplets_in<T> in{ri, ci, v, cb};
+  auto hk = dg.bits == 8u ? radix_hist_kernel<true, 8, triplets_in<T>> : radix_hist_kernel<true, 9, triplets_in<T>>;
+  hk<<<std::min(kKeyBlocks, blocks_for(nnz, 4u * kThreads)), kThreads, 0, st>>>(nnz, in, rows, cols, dg.passes, R.hist,
+                                                                                err);
+  CV_TRY(cudaGetLastError(), "radix_hist_kernel");
   uint32_t h_err[4];
   CV_TRY(cudaMemcpyAsync(h_err, err, sizeof(h_err), cudaMemcpyDeviceToHost, st), "cudaMemcpyAsync");
   CV_TRY(cudaStreamSynchronize(st), "cudaStreamSynchronize");
   if (h_err[0] & 1u) return fail(MFP_ERROR_INVALID_VALUE, "row id >= rows %u at element %u", rows, h_err[1]);
   if (h_err[0] & 2u) return fail(MFP_ERROR_INVALID_VALUE, "col id >= cols %u at element %u", cols, h_err[1]);
-  // not in CSR order: stable sort on (row, col); in order already, a stable sort would keep it
-  if (h_err[2] && (s = radix_sort_pairs<T>(nnz, rb + cb, k0, p0, sc))) return s;
-  rowptr_from_keys_kernel<<<blocks_for((uint64_t)nnz + 1, kThreads), kThreads, 0, st>>>(nnz, rows, k0, cb, rp);
-  csr_split_kernel<T><<<blocks_for(nnz, kThreads), kThreads, 0, st>>>(nnz, k0, p0, (1ull << cb) - 1ull, co, data);
-  CV_TRY(cudaGetLastError(), "csr_split_kernel");
+  const uint32_t *sorted_rows = ri;
+  if (!h_err[2]) {  // in CSR order already: a stable sort would keep it
+    csr_copy_kernel<T><<<blocks_for(nnz, kThreads), kThreads, 0, st>>>(nnz, ci, v, co, data);
+  } else {
+    unsigned long long *k[2] = {nullptr, nullptr};
+    T *p[2] = {nullptr, nullptr};
+    uint32_t *out_rows = nullptr;
+    for (uint32_t b = 0; b < 2u && b + 1u < dg.passes; ++b)
+      if ((s = sc.get(&k[b], nnz)) || (s = sc.get(&p[b], nnz))) return s;
+    // the last pass leaves the rows in the key buffer that it does not read
+    out_rows = reinterpret_cast<uint32_t *>(k[(dg.passes - 1u) & 1u]);
+    if (!out_rows && (s = sc.get(&out_rows, nnz))) return s;
+    const csr_out<T> out{out_rows, co, data, cb};
+    for (uint32_t pass = 0; pass < dg.passes; ++pass) {
+      const bool first = pass == 0, last = pass + 1u == dg.passes;
+      const pairs_in<T> mid_in{k[(pass + 1u) & 1u], p[(pass + 1u) & 1u]};
+      const pairs_out<T> mid_out{k[pass & 1u], p[pass & 1u]};
+      if (first)
+        s = last ? radix_pass<T>(nnz, in, out, dg, pass, R, err, sc) : radix_pass<T>(nnz, in, mid_out, dg, pass, R, err, sc);
+      else
+        s = last ? radix_pass<T>(nnz, mid_in, out, dg, pass, R, err, sc)
+                 : radix_pass<T>(nnz, mid_in, mid_out, dg, pass, R, err, sc);
+      if (s) return s;
+    }
+    sorted_rows = out_rows;
+  }
+  rowptr_from_rows_kernel<<<blocks_for((uint64_t)nnz + 1, kThreads), kThreads, 0, st>>>(nnz, rows, sorted_rows, rp);
+  CV_TRY(cudaGetLastError(), "rowptr_from_rows_kernel");
+  CV_TRY(cudaMemcpyAsync(h_err, err, sizeof(h_err), cudaMemcpyDeviceToHost, st), "cudaMemcpyAsync");
   CV_TRY(cudaStreamSynchronize(st), "cudaStreamSynchronize");
+  if (h_err[3]) return radix_error(h_err[3]);
   return ok();
 }
 

@@ -106,3 +106,29 @@ def test_scoo_tiles_on_two_streams_and_in_a_graph():
     dm.close()
     for w, y in zip(want, ys):
         assert np.array_equal(w.view(np.uint32), y.cpu().numpy().view(np.uint32))
+
+
+TILE = 6144  # keys per tile of the triplet sort
+
+
+@pytest.mark.parametrize("n", [1, 31, 33, TILE - 1, TILE, TILE + 1, 40 * TILE + 17])
+@pytest.mark.parametrize("rows, cols", [(2, 1), (1, 200), (3, 300), (500, 509), (70_000, 65_537), (1 << 20, 1 << 12),
+                                        (1 << 24, 0xFFFFFFFF)])
+def test_triplet_sort_digits_and_tiles(n, rows, cols):
+    """CSR from triplets equals a stable host sort: element counts around the
+    sort's tiles, key widths of 1 to 56 bits (1 to 7 digits of 8 or 9 bits,
+    digits that straddle the key's halves), repeated entries in input order."""
+    from matrix_format_performance_b200 import convert
+    rng = np.random.default_rng(n + rows)
+    r = rng.integers(0, rows, n).astype(np.uint32)
+    c = rng.integers(0, cols, n, dtype=np.uint64).astype(np.uint32)
+    r[n // 2:] = r[: n - n // 2]  # repeats
+    c[n // 2:] = c[: n - n // 2]
+    v = np.arange(n, dtype=np.float64)
+    rp, co, d = convert.csr_from_coo(rows, cols, dev(r.view(np.int32)), dev(c.view(np.int32)), dev(v), dtype=torch.float64)
+    order = np.lexsort((np.arange(n), c, r))
+    want = np.zeros(rows + 1, np.int64)
+    np.add.at(want, r.astype(np.int64) + 1, 1)
+    assert np.array_equal(rp.cpu().numpy(), np.cumsum(want))
+    assert np.array_equal(co.cpu().numpy().view(np.uint32), c[order])
+    assert np.array_equal(d.cpu().numpy(), v[order])
