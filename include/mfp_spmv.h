@@ -230,7 +230,9 @@ int mfp_dev_scratch_release(void);
  * gpu_matrix_multiplier.cu:22-43), 1 = CSR vector (a lane group per row;
  * csr_spmv_vector_kernel, :331-362), 2 = CSR-Adaptive (row bins;
  * csr_adaptive_spmv.cu:26-178).  Rows longer than long_row_threshold are
- * split across CTAs; rows longer than 4096 accumulate in FP64. */
+ * split across CTAs; rows longer than 4096 accumulate in FP64.  Without a
+ * configuration, row blocks without a row above 64 elements are read straight
+ * from global memory by lane groups (scalar still adds each row in CSR order). */
 typedef enum mfp_csr_algo { MFP_CSR_SCALAR = 0, MFP_CSR_VECTOR = 1, MFP_CSR_ADAPTIVE = 2 } mfp_csr_algo;
 typedef struct mfp_csr_config {
   uint32_t long_row_threshold; /* 0 = default for the algo; UINT32_MAX = never split */

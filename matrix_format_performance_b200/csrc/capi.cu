@@ -187,12 +187,14 @@ struct mfp_csr_plan {
   double *partials = nullptr;
   uint32_t *counters = nullptr;
   uint32_t *row_blocks = nullptr;
-  uint32_t *order = nullptr;  // work items heaviest first (n_main + n_pieces)
+  uint32_t *order = nullptr;  // work items heaviest first
+  uint32_t n_order = 0;       // n_main + n_pieces; direct plans: the items left to csr_kernel
   // warp-tile kernel (CSR vector on short rows): the row of the element before
   // each 256-element tile, and the COO-style workspace of the fix-up pass
   uint4 *blk = nullptr;  // per row block: element range and flags (see csr_args::blk)
   bool fast = false;     // row blocks without long rows start their loads before the row_ptr barrier
   bool binned = false;   // CSR scalar on the CSR-Adaptive bins, one thread per row
+  bool direct = false;   // rows straight from global memory (csr_direct_kernel)
   bool tile = false;
   uint32_t *tile_prev = nullptr;
   void *tile_ws = nullptr;
@@ -203,6 +205,9 @@ struct mfp_csr_plan {
 // Launch the CSR family's work items heaviest first (1) or in index order (0).
 #ifndef MFP_CSR_ORDER
 #define MFP_CSR_ORDER 1
+#endif
+#ifndef MFP_CSR_DIRECT
+#define MFP_CSR_DIRECT 1
 #endif
 
 namespace {
@@ -226,8 +231,44 @@ d::coo_carry<T> carries(void *ws, uint32_t warp_tiles) {
   cw.tail_row = cw.flags + warp_tiles;
   return cw;
 }
+bool auto_config(const mfp_csr_config *c) {
+  const mfp_csr_config none{};
+  return !c || memcmp(c, &none, sizeof(none)) == 0;
+}
 constexpr uint32_t kDefaultLong = 4096;
+constexpr uint32_t kDirectMixed = 16u << 20;
 constexpr uint32_t kDefaultAssist = 64;
+
+// Row blocks of 256 rows: element range and, in z, bit 0 a long row, bit 1 an
+// assisted row, bits 8-15 the lanes per row of csr_direct_kernel with FP32
+// values (a power of two, at least 3/4 of the mean number of aligned quads a row
+// touches: one or two passes), bits 16-23 with FP64 values (at least half).
+// Fewer lanes let a warp span more rows, whose x gathers share cache lines, but
+// a pass should read whole 128-byte lines of the values: the FP32 banded matrix
+// with 8 lanes (128 bytes) ran 378 us on 8M rows and with 4 lanes 485, which
+// fetch a line's halves at different times; in FP64 (4M rows) 4 lanes ran 274 us
+// and 8 lanes 298.  *regular = elements in blocks without either.
+std::vector<uint4> row_block_info(uint32_t rows, const uint32_t *rp, uint32_t long_thr, uint32_t assist_thr,
+                                  uint64_t *regular) {
+  std::vector<uint4> br(ceil_div(rows, d::kBlock));
+  *regular = 0;
+  for (uint32_t b = 0; b < br.size(); ++b) {
+    const uint32_t r0 = b * d::kBlock, r1 = std::min(rows, r0 + d::kBlock);
+    uint32_t flags = 0, quads = 0;
+    for (uint32_t r = r0; r < r1; ++r) {
+      const uint32_t len = rp[r + 1] - rp[r];
+      if (len > long_thr) flags |= 1u;
+      else if (len > assist_thr) flags |= 2u;
+      if (len) quads += (rp[r + 1] + 3u) / 4u - rp[r] / 4u;
+    }
+    uint32_t g32 = 2, g64 = 2;
+    while (g32 < 16u && 4ull * g32 * (r1 - r0) < 3ull * quads) g32 *= 2;
+    while (g64 < 16u && 4ull * g64 * (r1 - r0) < 2ull * quads) g64 *= 2;
+    if (!flags) *regular += rp[r1] - rp[r0];
+    br[b] = make_uint4(rp[r0], rp[r1], flags | (g32 << 8) | (g64 << 16), 0u);
+  }
+  return br;
+}
 // One CTA per long row up to 65,536 elements: on the power-law matrix (rows
 // up to 50,000) pieces of 4,096 / 16,384 / 65,536 elements took CSR scalar
 // to 0.191 / 0.188 / 0.184 ms and CSR-Adaptive to 0.172 / 0.168 / 0.164 ms
@@ -351,6 +392,7 @@ extern "C" int mfp_csr_plan_create(uint32_t rows, uint32_t cols, uint32_t nnz, c
   int st = check_row_ptr(rows, nnz, rp);
   if (st) return st;
   mfp_csr_config cfg = config ? *config : mfp_csr_config{};
+  const bool automatic = auto_config(config);
   auto *plan = new mfp_csr_plan();
   cudaGetDevice(&plan->device);
   plan->algo = algo;
@@ -367,7 +409,25 @@ extern "C" int mfp_csr_plan_create(uint32_t rows, uint32_t cols, uint32_t nnz, c
   // 27-point stencil, banded 8M) a bin holds too few rows for its threads.
   const bool exact = cfg.long_row_threshold == UINT32_MAX && cfg.assist_threshold == UINT32_MAX;
   plan->binned = algo == MFP_CSR_SCALAR && cfg.kernel == 0 && !exact && rows && (double)nnz / rows < 16.0;
-  if (algo == MFP_CSR_ADAPTIVE || plan->binned)
+  // Automatic plans with nearly all elements, or half of many, in row blocks
+  // without a row above 64 elements: those rows straight from global memory, the
+  // others in the CSR-Adaptive bins beside them (two launches: 64 uneven matrices
+  // of 72M nonzeros 249 -> 230 us, 40 of 36M 123 -> 113, but 14 of 8M 32.4 -> 34.7
+  // and 20 of 15M in FP64 74 -> 82).  B200 against the row blocks / bins / warp
+  // tiles, inputs changing from pass to pass: banded 8M rows FP32 scalar 400 ->
+  // 361 us, vector 539 -> 341, 4M rows FP64 scalar 351 -> 275; 27-point 128^3 FP32
+  // scalar 121 -> 107, Adaptive 135 -> 97, 101^3 FP64 vector 96 -> 73; 5-point
+  // 1000^2 FP64 vector 27.5 -> 21; uniform 500k rows FP32 91 -> 79.  A power-law
+  // matrix has a row above 64 elements in nine blocks of ten and keeps its
+  // kernels.
+  std::vector<uint4> blk;
+  if (MFP_CSR_DIRECT && automatic && nnz) {
+    uint64_t regular = 0;
+    blk = row_block_info(rows, rp, kDefaultLong, kDefaultAssist, &regular);
+    plan->direct = 16 * regular >= 15ull * nnz || (2 * regular >= nnz && nnz >= kDirectMixed);
+    if (plan->direct) plan->binned = false;
+  }
+  if (algo == MFP_CSR_ADAPTIVE || plan->binned || plan->direct)
     cfg.bin_nnz = cfg.bin_nnz ? std::min(cfg.bin_nnz, kMaxBin) : kMaxBin;
   if (algo == MFP_CSR_ADAPTIVE) {
     // rows longer than a bin and up to 4096 elements: one CTA each (plain
@@ -382,7 +442,7 @@ extern "C" int mfp_csr_plan_create(uint32_t rows, uint32_t cols, uint32_t nnz, c
     // share rows through the segmented scan.  Measured on B200 against 2 and 4
     // lanes per row: power-law 4M 0.187 ms (2 lanes 0.240), 27-point stencil
     // 0.153 ms (0.178), banded 8M 0.599 ms (0.669), FP32.
-    plan->tile = L == 0 && cfg.kernel == 0 && rows && (double)nnz / rows < 64.0;
+    plan->tile = L == 0 && cfg.kernel == 0 && rows && (double)nnz / rows < 64.0 && !plan->direct;
     if (L == 0) {
       // Measured on B200 over 2,200 seeded matrices (uniform, Zipf, banded,
       // block-diagonal, stencil, dense-row families) and the 4M-row power-law
@@ -427,14 +487,19 @@ extern "C" int mfp_csr_plan_create(uint32_t rows, uint32_t cols, uint32_t nnz, c
     ++nlong;
   }
   std::vector<uint32_t> blocks;
-  if (algo == MFP_CSR_ADAPTIVE || plan->binned) {
+  // (direct plans: bins of the rows that csr_direct_kernel leaves out, and of the
+  // others for unaligned arrays; a bin does not cross the two kinds of blocks)
+  const bool bins = algo == MFP_CSR_ADAPTIVE || plan->binned || plan->direct;
+  auto left_out = [&](uint32_t r) { return !plan->direct || (blk[r / d::kBlock].z & 3u); };
+  if (bins) {
     blocks.push_back(0);
     uint32_t cur_rows = 0, cur_nnz = 0;
     const uint32_t max_rows = 4 * d::kBlock;
     for (uint32_t r = 0; r < rows; ++r) {
       const uint32_t len = rp[r + 1] - rp[r];
       const bool own = len > cfg.long_row_threshold || len > cfg.bin_nnz;
-      if (cur_rows && (own || cur_nnz + len > cfg.bin_nnz || cur_rows >= max_rows)) {
+      if (cur_rows && (own || cur_nnz + len > cfg.bin_nnz || cur_rows >= max_rows ||
+                       (r % d::kBlock == 0 && left_out(r) != left_out(r - 1)))) {
         blocks.push_back(r);
         cur_rows = cur_nnz = 0;
       }
@@ -462,12 +527,14 @@ extern "C" int mfp_csr_plan_create(uint32_t rows, uint32_t cols, uint32_t nnz, c
     delete plan;
     return fail(MFP_ERROR_TOO_LARGE, "grid too large");
   }
-  // launch order: work items by element count, heaviest first (stable)
-  std::vector<uint32_t> order((size_t)plan->n_main + plan->n_pieces);
+  // launch order: work items by element count, heaviest first (stable); of a
+  // direct plan only those that csr_direct_kernel leaves out
+  std::vector<uint32_t> order;
   {
-    std::vector<uint64_t> cost(order.size());
+    const uint32_t items = plan->n_main + plan->n_pieces;
+    std::vector<uint64_t> cost(items);
     for (uint32_t b = 0; b < plan->n_main; ++b) {
-      const bool bins = algo == MFP_CSR_ADAPTIVE || plan->binned;
+      if (bins && !left_out(blocks[b])) continue;
       const uint32_t r0 = bins ? blocks[b] : b * d::kBlock;
       const uint32_t r1 = bins ? blocks[b + 1] : std::min(rows, r0 + d::kBlock);
       uint64_t c = r1 - r0;
@@ -476,11 +543,15 @@ extern "C" int mfp_csr_plan_create(uint32_t rows, uint32_t cols, uint32_t nnz, c
         if (len <= cfg.long_row_threshold) c += len;
       }
       cost[b] = c;
+      order.push_back(b);
     }
-    for (uint32_t k = 0; k < plan->n_pieces; ++k) cost[plan->n_main + k] = pieces[k].e1 - pieces[k].e0;
-    for (uint32_t i = 0; i < order.size(); ++i) order[i] = i;
+    for (uint32_t k = 0; k < plan->n_pieces; ++k) {
+      cost[plan->n_main + k] = pieces[k].e1 - pieces[k].e0;
+      order.push_back(plan->n_main + k);
+    }
     std::stable_sort(order.begin(), order.end(), [&](uint32_t a, uint32_t b) { return cost[a] > cost[b]; });
   }
+  plan->n_order = (uint32_t)order.size();
   if ((st = upload(&plan->order, order.data(), order.size(), &plan->device_bytes)) ||
       (st = upload(&plan->pieces, pieces.data(), pieces.size(), &plan->device_bytes)) ||
       (st = dmalloc(&plan->partials, slots, &plan->device_bytes)) ||
@@ -491,26 +562,14 @@ extern "C" int mfp_csr_plan_create(uint32_t rows, uint32_t cols, uint32_t nnz, c
   }
   // row blocks that start their loads before the row_ptr barrier: measured
   // faster for lanes per row and for long rows (mean length 16 and up)
-  plan->fast = algo != MFP_CSR_ADAPTIVE && (algo == MFP_CSR_VECTOR || (rows && (double)nnz / rows >= 16.0));
+  plan->fast = !plan->direct && algo != MFP_CSR_ADAPTIVE && (algo == MFP_CSR_VECTOR || (rows && (double)nnz / rows >= 16.0));
   if (plan->fast) {
-    // per row block: its element range and whether it holds a long or an
-    // assisted row
-    std::vector<uint4> br(plan->n_main);
-    for (uint32_t b = 0; b < plan->n_main; ++b) {
-      const uint32_t r0 = b * d::kBlock;
-      const uint32_t r1 = std::min(rows, r0 + d::kBlock);
-      uint32_t flags = 0;
-      for (uint32_t r = r0; r < r1; ++r) {
-        const uint32_t len = rp[r + 1] - rp[r];
-        if (len > cfg.long_row_threshold) flags |= 1u;
-        else if (len > plan->assist_thr) flags |= 2u;
-      }
-      br[b] = make_uint4(rp[r0], rp[r1], flags, 0u);
-    }
-    if ((st = upload(&plan->blk, br.data(), br.size(), &plan->device_bytes))) {
-      mfp_csr_plan_destroy(plan);
-      return st;
-    }
+    uint64_t regular = 0;
+    blk = row_block_info(rows, rp, cfg.long_row_threshold, plan->assist_thr, &regular);
+  }
+  if ((plan->fast || plan->direct) && (st = upload(&plan->blk, blk.data(), blk.size(), &plan->device_bytes))) {
+    mfp_csr_plan_destroy(plan);
+    return st;
   }
   if (plan->tile) {
     // the row holding element 256 w - 1, for every warp tile w > 0
@@ -590,6 +649,31 @@ template <typename T>
 int csr_tile_spmv(const mfp_csr_plan *plan, const T *data, const uint32_t *cols, const uint32_t *rp, const T *x,
                   T *y, cudaStream_t s);
 
+// Launches that follow another launch of the same call may start early
+// (programmatic dependent launch): their CTAs are placed while the preceding
+// kernel drains and wait for it in griddep_wait() before touching its output.
+#ifndef MFP_PDL
+#define MFP_PDL 1
+#endif
+template <typename... KArgs, typename... Args>
+cudaError_t launch_after(void (*k)(KArgs...), uint32_t grid, cudaStream_t s, Args &&...args) {
+  if (!MFP_PDL) {
+    k<<<grid, d::kBlock, 0, s>>>(std::forward<Args>(args)...);
+    return cudaGetLastError();
+  }
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(d::kBlock);
+  cfg.dynamicSmemBytes = 0;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, k, std::forward<Args>(args)...);
+}
+
 template <typename T>
 int csr_spmv(const mfp_csr_plan *plan, const T *data, const uint32_t *cols, const uint32_t *rp, const T *x,
              T *y, void *stream) {
@@ -598,6 +682,7 @@ int csr_spmv(const mfp_csr_plan *plan, const T *data, const uint32_t *cols, cons
   if (!rp || !y || (plan->nnz && (!data || !cols || !x))) return fail(MFP_ERROR_INVALID_VALUE, "null device array");
   d::csr_args<T> A{};
   A.n_rows = plan->rows;
+  A.nnz = plan->nnz;
   A.row_ptr = rp;
   A.cols = cols;
   A.vals = data;
@@ -650,12 +735,30 @@ int csr_spmv(const mfp_csr_plan *plan, const T *data, const uint32_t *cols, cons
   if (plan->tile && !exact_order) return csr_tile_spmv<T>(plan, data, cols, rp, x, y, s);
   const uint32_t grid = plan->n_main + plan->n_pieces;
   if (grid == 0) return ok();
-#define MFP_CSR_LAUNCH(ALGO, FAST)                                                   \
+#define MFP_CSR_LAUNCH_N(ALGO, FAST, N)                                              \
   if (vec)                                                                           \
-    d::csr_kernel<T, ALGO, true, FAST><<<grid, d::kBlock, 0, s>>>(A);                \
+    d::csr_kernel<T, ALGO, true, FAST><<<N, d::kBlock, 0, s>>>(A);                   \
   else                                                                               \
-    d::csr_kernel<T, ALGO, false, FAST><<<grid, d::kBlock, 0, s>>>(A);
+    d::csr_kernel<T, ALGO, false, FAST><<<N, d::kBlock, 0, s>>>(A);
+#define MFP_CSR_LAUNCH(ALGO, FAST) MFP_CSR_LAUNCH_N(ALGO, FAST, grid)
   const bool fast = plan->fast && plan->blk;
+  if (plan->direct) {
+    const bool seq = plan->algo == MFP_CSR_SCALAR;
+    if (!vec) A.order = nullptr;  // unaligned arrays: every bin
+    const uint32_t rest = vec ? plan->n_order : grid;
+    if (rest && seq) { MFP_CSR_LAUNCH_N(3, false, rest) }
+    if (rest && !seq) { MFP_CSR_LAUNCH_N(2, false, rest) }
+    if (vec) {
+      auto k = seq ? d::csr_direct_kernel<T, true> : d::csr_direct_kernel<T, false>;
+      if (rest) {  // beside the blocks with longer rows
+        const cudaError_t e = launch_after(k, ceil_div(plan->rows, d::kBlock), s, A);
+        if (e != cudaSuccess) return cuda_fail(e, "csr_direct_kernel launch");
+      } else {
+        k<<<ceil_div(plan->rows, d::kBlock), d::kBlock, 0, s>>>(A);
+      }
+    }
+    return check_launch("csr_direct_kernel launch");
+  }
   switch (plan->algo) {
     case 0:
       if (plan->binned) {
@@ -672,6 +775,7 @@ int csr_spmv(const mfp_csr_plan *plan, const T *data, const uint32_t *cols, cons
     default: MFP_CSR_LAUNCH(2, false) break;
   }
 #undef MFP_CSR_LAUNCH
+#undef MFP_CSR_LAUNCH_N
   return check_launch("csr_kernel launch");
 }
 
@@ -698,30 +802,6 @@ int fill(uint64_t n, T *v, T value, void *stream) {
   return check_launch("fill_kernel launch");
 }
 
-// Launches that follow another launch of the same call may start early
-// (programmatic dependent launch): their CTAs are placed while the preceding
-// kernel drains and wait for it in griddep_wait() before touching its output.
-#ifndef MFP_PDL
-#define MFP_PDL 1
-#endif
-template <typename... KArgs, typename... Args>
-cudaError_t launch_after(void (*k)(KArgs...), uint32_t grid, cudaStream_t s, Args &&...args) {
-  if (!MFP_PDL) {
-    k<<<grid, d::kBlock, 0, s>>>(std::forward<Args>(args)...);
-    return cudaGetLastError();
-  }
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(grid);
-  cfg.blockDim = dim3(d::kBlock);
-  cfg.dynamicSmemBytes = 0;
-  cfg.stream = s;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, k, std::forward<Args>(args)...);
-}
 
 
 template <typename T, bool ACCUM = false>
@@ -1971,6 +2051,8 @@ int mfp_matrix_get_info(const mfp_matrix *m, mfp_matrix_info *out) {
     out->kernel_launches = 1u + (m->coo_nnz ? (m->coo_nnz > d::kWarpTile ? 2u : 1u) : 0u);
   else if ((m->plan && m->plan->tile) || (m->tiles && m->rows))  // warp-tile CSR, row-ordered SCOO: tiles + fix-up
     out->kernel_launches = 2u;
+  else if (m->plan && m->plan->direct)  // the blocks with longer rows are a second launch
+    out->kernel_launches = m->plan->n_order ? 2u : 1u;
   else
     out->kernel_launches = 1u;
   return ok();

@@ -267,6 +267,9 @@ __device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t v, uint32_t *s
 // stream has completed and its writes are visible (a no-op when the launch did
 // not allow early start).  Hardware-managed; not a poll on memory.
 __device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// Lets the next kernel of the stream start (if its launch allows it) once every
+// CTA of this one has got here or ended.
+__device__ __forceinline__ void griddep_launch() { asm volatile("griddepcontrol.launch_dependents;"); }
 
 }  // namespace dev
 }  // namespace mfp

@@ -671,7 +671,7 @@ __device__ __forceinline__ void run_piece(const long_piece &pc, const T *__restr
 // ---------------------------------------------------------------------------
 template <typename T>
 struct csr_args {
-  uint32_t n_rows;
+  uint32_t n_rows, nnz;
   const uint32_t *__restrict__ row_ptr;
   const uint32_t *__restrict__ cols;
   const T *__restrict__ vals;
@@ -974,6 +974,7 @@ __device__ __forceinline__ void csr_adaptive_main(const csr_args<T> &A, csr_smem
 template <typename T, int ALGO, bool VEC, bool FAST = false>
 __global__ void __launch_bounds__(kBlock, sizeof(T) == 4 ? (ALGO != 1 ? MFP_CSR_MINBLOCKS : MFP_CSR_MINBLOCKS_VEC) : (ALGO == 0 ? MFP_CSR_MINBLOCKS64 : MFP_CSR_MINBLOCKS64_OTHER)) csr_kernel(const csr_args<T> A) {
   __shared__ csr_smem<T> sm;
+  griddep_launch();  // csr_direct_kernel runs beside this one
   const uint64_t pol = policy_evict_first();
   // the hardware starts blocks in index order: with A.order the heaviest work
   // items (by element count) start first, which shortens the tail; without
@@ -995,6 +996,133 @@ __global__ void __launch_bounds__(kBlock, sizeof(T) == 4 ? (ALGO != 1 ? MFP_CSR_
     csr_adaptive_main<T, VEC, ALGO == 3>(A, sm, pol, b);
   else
     csr_rowblock_main<T, ALGO, VEC, FAST>(A, sm, pol, b);
+}
+
+// ---------------------------------------------------------------------------
+// CSR rows straight from global memory: row blocks whose rows are all short
+// (at most 64 elements).  A group of G lanes takes a row, lane l the aligned
+// quads of elements l, l + G, ... (one 16-byte load of column ids and one 16- or
+// 32-byte load of values each, coalesced over the warp's rows); no shared
+// memory and no barriers.  SEQ (CSR scalar): the products are added one after
+// the other in CSR order, the running sum handed from lane to lane, so a row's
+// bits are those of one thread summing it.  Otherwise (CSR vector, Adaptive)
+// each lane adds its own products and a shuffle tree the lanes' sums.
+// Staging the products through shared memory instead, and the 8-element lane
+// groups of the warp-tile kernel, spend the L1 data path on it: 10.6 wavefronts
+// per 32 nonzeros on the banded matrix, 65% of the L1 rate with DRAM at 79%.
+// Here the banded matrix (8M rows, FP32: 341 us summed by trees, 361 in order) is
+// at 100% and 95% of the DRAM rate; the 27-point stencil (128^3: 97 and 107 us)
+// spends its L1 wavefronts on the gathers, 8 cache lines for 32 lanes.
+// ---------------------------------------------------------------------------
+template <typename T>
+struct row_quad {
+  T v[4];
+  uint32_t c[4];
+  uint32_t e;  // first element; elements outside [rs, re) are masked
+};
+template <typename T>
+__device__ __forceinline__ void load_quad(const csr_args<T> &A, uint32_t e, uint32_t re, row_quad<T> &q, uint64_t pol) {
+  q.e = e;
+  if (e >= re) return;
+  if (e + 4u <= A.nnz) {
+    ld_stream4(A.vals + e, q.v, pol);
+    ld_stream4(A.cols + e, q.c, pol);
+  } else {
+#pragma unroll
+    for (uint32_t j = 0; j < 4; ++j)
+      if (e + j < A.nnz) {
+        q.v[j] = ld_stream1(A.vals + e + j, pol);
+        q.c[j] = ld_stream1(A.cols + e + j, pol);
+      }
+  }
+}
+// The quad's products, 0 outside the row.
+template <typename T>
+__device__ __forceinline__ void quad_products(const csr_args<T> &A, const row_quad<T> &q, uint32_t rs, uint32_t re,
+                                              T (&p)[4]) {
+  T xv[4];
+#pragma unroll
+  for (uint32_t j = 0; j < 4; ++j) {
+    const bool on = q.e + j >= rs && q.e + j < re;
+    xv[j] = on ? ld_x(A.x + q.c[j]) : T(0);
+  }
+#pragma unroll
+  for (uint32_t j = 0; j < 4; ++j) {
+    const bool on = q.e + j >= rs && q.e + j < re;
+    p[j] = on ? mul_rn(q.v[j], xv[j]) : T(0);
+  }
+}
+
+template <typename T, bool SEQ, int G>
+__device__ __forceinline__ void csr_rows_direct(const csr_args<T> &A, uint64_t pol, uint32_t r0, uint32_t nr) {
+  constexpr uint32_t kRows = 32u / G;  // rows side by side; a warp's 32 rows take G rounds
+  const uint32_t lane = threadIdx.x & 31u, w0 = threadIdx.x & ~31u, gl = lane % G;
+  if (w0 >= nr) return;
+  const uint32_t end = r0 + nr;
+  const uint32_t p0 = __ldg(A.row_ptr + min(r0 + w0 + lane, end));
+  const uint32_t p1 = __ldg(A.row_ptr + min(r0 + w0 + lane + 1u, end));
+  T out = T(0);
+#pragma unroll 1
+  for (uint32_t s = 0; s < (uint32_t)G; ++s) {
+    const uint32_t src = s * kRows + lane / G;
+    const uint32_t rs = __shfl_sync(0xffffffffu, p0, src), re = __shfl_sync(0xffffffffu, p1, src);
+    row_quad<T> q;
+    load_quad(A, (rs & ~3u) + 4u * gl, re, q, pol);
+    const uint32_t passes =
+        __reduce_max_sync(0xffffffffu, rs < re ? (re - (rs & ~3u) + 4u * G - 1u) / (4u * G) : 0u);
+    T acc = T(0);
+    for (uint32_t k = 0; k < passes; ++k) {
+      T p[4];
+      quad_products(A, q, rs, re, p);
+      if (k + 1u < passes) load_quad(A, q.e + 4u * G, re, q, pol);
+      if (SEQ) {
+#pragma unroll
+        for (int l = 0; l < G; ++l) {  // lane l's turn: the others' values are dropped
+          const T t = add_rn(add_rn(add_rn(add_rn(acc, p[0]), p[1]), p[2]), p[3]);
+          acc = __shfl_sync(0xffffffffu, t, l, G);
+        }
+      } else {
+        acc = add_rn(add_rn(add_rn(add_rn(acc, p[0]), p[1]), p[2]), p[3]);
+      }
+    }
+    if (!SEQ) acc = group_reduce_down(acc, G);
+    // row i of the warp goes to lane i
+    const T r = __shfl_sync(0xffffffffu, acc, (lane * G) & 31u);
+    if (lane / kRows == s) out = r;
+  }
+  if (w0 + lane < nr) A.y[r0 + w0 + lane] = out;
+}
+
+// CTAs per SM the kernel is register-limited to (FP32, FP64).  Warps in flight
+// count for more than loads per warp: with two rounds of rows in flight per warp
+// at 5 CTAs (FP64: 4) the banded matrix took 378 us, here 361.
+#ifndef MFP_DIRECT_MINBLOCKS
+#define MFP_DIRECT_MINBLOCKS 8
+#endif
+#ifndef MFP_DIRECT_MINBLOCKS64
+#define MFP_DIRECT_MINBLOCKS64 6
+#endif
+// Row blocks in the plan's blk flags: bits 0 and 1 as in csr_args::blk, bits
+// 8-15 the lanes per row (FP32), bits 16-23 (FP64).  Blocks with a longer row and the long rows' pieces are
+// a csr_kernel launch of their own (their registers would weigh on this one),
+// which comes first and which this one runs beside: the two write different
+// rows.  Block 0's wait at the end keeps this kernel from completing, and so the
+// stream from going on, before that one (one block is enough; waiting blocks
+// hold their place on an SM).
+template <typename T, bool SEQ>
+__global__ void __launch_bounds__(kBlock, sizeof(T) == 4 ? MFP_DIRECT_MINBLOCKS : MFP_DIRECT_MINBLOCKS64)
+    csr_direct_kernel(const csr_args<T> A) {
+  const uint64_t pol = policy_evict_first();
+  const uint32_t flags = __ldg(&A.blk[blockIdx.x].z);
+  const uint32_t r0 = blockIdx.x * kBlock, nr = min((uint32_t)kBlock, A.n_rows - r0);
+  switch (flags & 3u ? 0u : (sizeof(T) == 4 ? flags >> 8 : flags >> 16) & 0xffu) {
+    case 0: break;
+    case 2: csr_rows_direct<T, SEQ, 2>(A, pol, r0, nr); break;
+    case 4: csr_rows_direct<T, SEQ, 4>(A, pol, r0, nr); break;
+    case 8: csr_rows_direct<T, SEQ, 8>(A, pol, r0, nr); break;
+    default: csr_rows_direct<T, SEQ, 16>(A, pol, r0, nr); break;
+  }
+  if (blockIdx.x == 0) griddep_wait();
 }
 
 // ---------------------------------------------------------------------------

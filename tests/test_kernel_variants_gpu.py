@@ -132,3 +132,57 @@ def test_triplet_sort_digits_and_tiles(n, rows, cols):
     assert np.array_equal(rp.cpu().numpy(), np.cumsum(want))
     assert np.array_equal(co.cpu().numpy().view(np.uint32), c[order])
     assert np.array_equal(d.cpu().numpy(), v[order])
+
+
+NEVER = 0xFFFFFFFF
+
+
+def short_lengths(case):
+    rng = np.random.default_rng(21)
+    if case == "two_lanes":       # 0 to 9 elements: 2 lanes per row
+        return rng.integers(0, 10, 1001)
+    if case == "sixteen_lanes":   # up to 64 elements, several passes; a last block of one row
+        return np.concatenate([rng.integers(40, 65, 512), [64]])
+    if case == "growing":         # every lane count, the last row ends the array inside a quad
+        return np.concatenate([np.arange(65).repeat(40), [3]])
+    lens = rng.integers(20, 40, 20 * 4096)  # mixed: blocks with longer rows between blocks without
+    lens[300], lens[301], lens[1500], lens[3000:3010], lens[-1] = 65, 4_097, 20_000, 3_000, 66
+    return lens
+
+
+@pytest.mark.parametrize("case", ["two_lanes", "sixteen_lanes", "growing", "mixed"])
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+def test_csr_short_rows_straight_from_memory(oracle_lib, case, dtype):
+    """CSR plans without a configuration read row blocks of short rows straight
+    from global memory.  CSR scalar keeps the bits of the exact-order setting
+    (one thread per row) on rows up to 64 elements; every algorithm is within
+    tolerance, also on arrays that are not 16-byte aligned."""
+    from matrix_format_performance_b200.device import CSR_ADAPTIVE, CSR_SCALAR, CSR_VECTOR
+    m = csr(short_lengths(case), 3_000, dtype)
+    x = synth.vector(6, m.cols).astype(dtype)
+    exact = DeviceMatrix.from_csr(m, CSR_SCALAR, {"long_row_threshold": NEVER, "assist_threshold": NEVER})
+    want = spmv(exact, m, x)
+    exact.close()
+    short = np.diff(m.row_ptr.astype(np.int64)) <= 64
+    sfx = "f32" if dtype == np.float32 else "f64"
+    for fmt in (CSR_SCALAR, CSR_VECTOR, CSR_ADAPTIVE):
+        dm = DeviceMatrix.from_csr(m, fmt)
+        assert dm.info().kernel_launches == (2 if case == "mixed" else 1)
+        y = spmv(dm, m, x)
+        assert np.array_equal(y.view(np.uint8), spmv(dm, m, x).view(np.uint8))
+        dm.close()
+        check(oracle_lib, m, x, y, f"{case} {fmt}")
+        if fmt == CSR_SCALAR:
+            assert np.array_equal(y[short].view(np.uint8), want[short].view(np.uint8))
+        plan = C.c_void_p()
+        rp_host = np.ascontiguousarray(m.row_ptr)
+        call("mfp_csr_plan_create", m.rows, m.cols, m.nnz, C.c_void_p(rp_host.ctypes.data), fmt, None, C.byref(plan))
+        v = torch.zeros(m.nnz + 1, dtype=dev(m.data).dtype, device="cuda")
+        c = torch.zeros(m.nnz + 1, dtype=torch.int32, device="cuda")
+        v[1:], c[1:] = dev(m.data), dev(m.columns.view(np.int32))
+        rp, xt = dev(m.row_ptr.view(np.int32)), dev(x)
+        yt = torch.full((m.rows,), float("nan"), dtype=v.dtype, device="cuda")
+        call(f"mfp_csr_spmv_{sfx}", plan, p(v[1:]), p(c[1:]), p(rp), p(xt), p(yt), None)
+        torch.cuda.synchronize()
+        call("mfp_csr_plan_destroy", plan)
+        check(oracle_lib, m, x, yt.cpu().numpy(), f"unaligned {case} {fmt}")
