@@ -272,8 +272,13 @@ std::vector<uint4> row_block_info(uint32_t rows, const uint32_t *rp, uint32_t lo
 // One CTA per long row up to 65,536 elements: on the power-law matrix (rows
 // up to 50,000) pieces of 4,096 / 16,384 / 65,536 elements took CSR scalar
 // to 0.191 / 0.188 / 0.184 ms and CSR-Adaptive to 0.172 / 0.168 / 0.164 ms
-// (each extra piece adds a CTA-wide FP64 reduction and the combine).
-constexpr uint32_t kDefaultPiece = 65536;
+// (each extra piece adds a CTA-wide FP64 reduction and the combine).  But a
+// piece of 50,000 elements takes its CTA 30 to 70 us, which is longer than a
+// small matrix's whole product should: pieces of nnz / 512 elements (at least
+// 2,048) keep a piece to a fraction of it.  Power-law 100k rows FP64 31 -> 12.6
+// us, 300k rows FP32 31.5 -> 17.9, 1M rows FP64 74 -> 50, 4M rows unchanged;
+// nnz / 1024 and nnz / 4096 were 0-4 us slower from 300k rows on.
+constexpr uint32_t kDefaultPiece = 65536, kMinPiece = 2048, kPieceShare = 512;
 constexpr uint32_t kFp64Rows = 4096;  // rows longer than this accumulate in FP64
 constexpr uint32_t kMaxBin = d::kChunk - 4;
 }  // namespace
@@ -399,7 +404,7 @@ extern "C" int mfp_csr_plan_create(uint32_t rows, uint32_t cols, uint32_t nnz, c
   plan->rows = rows;
   plan->cols = cols;
   plan->nnz = nnz;
-  if (cfg.piece_nnz == 0) cfg.piece_nnz = kDefaultPiece;
+  if (cfg.piece_nnz == 0) cfg.piece_nnz = std::min(kDefaultPiece, std::max(kMinPiece, (nnz / kPieceShare + 255u) & ~255u));
   cfg.piece_nnz = std::max(cfg.piece_nnz, 256u);
   // CSR scalar on short rows (mean length below 16, automatic kernel, not
   // the exact-order setting): the CSR-Adaptive bins, which balance elements
