@@ -784,17 +784,27 @@ int csr_spmv(const mfp_csr_plan *plan, const T *data, const uint32_t *cols, cons
   return check_launch("csr_kernel launch");
 }
 
+constexpr uint32_t kEllVecRows = 600000;
 template <typename T>
 int ell_spmv(uint32_t rows, uint32_t width, const T *data, const uint32_t *cols, const T *x, T *y,
              void *stream) {
   if (rows == 0) return ok();
   if (!y || (width && (!data || !cols || !x))) return fail(MFP_ERROR_INVALID_VALUE, "null device array");
-  const bool vec = (rows % 4 == 0) && aligned16(data) && aligned16(cols) && aligned16(y);
+  // Four rows per thread with 16-byte loads: FP32 on matrices whose rows / 4
+  // threads fill the chip (27-point 128^3 70 us against 77 with a row per
+  // thread, banded 2M rows 76 against 80).  Smaller ones want the threads
+  // (27-point 60^3 20 us against 12, banded 200k rows FP64 31 against 15), and in
+  // FP64 a row per thread is as fast at every size (128^3 109 against 119).
+  const bool vec = sizeof(T) == 4 && rows >= kEllVecRows && rows % 4 == 0 && aligned16(data) && aligned16(cols) &&
+                   aligned16(y);
   cudaStream_t s = as_stream(stream);
-  if (vec)
-    d::ell_kernel<T, true><<<ceil_div(rows / 4, d::kBlock), d::kBlock, 0, s>>>(rows, width, data, cols, x, y);
-  else
-    d::ell_kernel<T, false><<<ceil_div(rows, d::kBlock), d::kBlock, 0, s>>>(rows, width, data, cols, x, y);
+  if constexpr (sizeof(T) == 4) {
+    if (vec) {
+      d::ell_kernel<T, 4, 4><<<ceil_div(rows / 4, d::kBlock), d::kBlock, 0, s>>>(rows, width, data, cols, x, y);
+      return check_launch("ell_kernel launch");
+    }
+  }
+  d::ell_kernel<T, 1, 8><<<ceil_div(rows, d::kBlock), d::kBlock, 0, s>>>(rows, width, data, cols, x, y);
   return check_launch("ell_kernel launch");
 }
 

@@ -186,3 +186,31 @@ def test_csr_short_rows_straight_from_memory(oracle_lib, case, dtype):
         torch.cuda.synchronize()
         call("mfp_csr_plan_destroy", plan)
         check(oracle_lib, m, x, yt.cpu().numpy(), f"unaligned {case} {fmt}")
+
+
+@pytest.mark.parametrize("width", [1, 2, 3, 7, 8, 9, 15, 64])
+@pytest.mark.parametrize("rows", [1, 255, 4_001, 600_000, 600_004])
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+def test_ell_widths_and_row_counts(width, rows, dtype):
+    """ELL on both sides of the row count from which a thread takes four rows,
+    at widths around the slots in flight: the bits of the slot loop in order,
+    padding included."""
+    from matrix_format_performance_b200.device import DeviceMatrix as D
+    if rows > 10_000 and width > 9:
+        rows = 600_000 // 4
+    rng = np.random.default_rng(width + rows)
+    cols = 777
+    e = F.ell_matrix_class.__new__(F.ell_matrix_class)
+    e.rows, e.cols, e.dtype, e.elements_in_rows = rows, cols, np.dtype(dtype), width
+    e.columns = rng.integers(0, cols, rows * width).astype(np.uint32)
+    e.data = rng.uniform(-1, 1, rows * width).astype(dtype)
+    e.data[rng.random(rows * width) < 0.1] = 0
+    x = rng.uniform(-1, 1, cols).astype(dtype)
+    dm = D.from_ell(e)
+    y = spmv(dm, e, x)
+    dm.close()
+    want = np.zeros(rows, dtype)
+    for k in range(width):
+        s = slice(k * rows, (k + 1) * rows)
+        want = want + e.data[s] * x[e.columns[s]]
+    assert np.array_equal(y.view(np.uint8), want.astype(dtype).view(np.uint8))
