@@ -1092,42 +1092,43 @@ int lowp_spmv(int vt, uint32_t rows, uint32_t nnz, const uint32_t *rp, const uin
   return check_launch("lowp_kernel launch");
 }
 
-// Runs of 8 consecutive x entries read with 16-byte loads where a lane's rows
-// share a column offset (1), or always 8 gathers (0).
-#ifndef MFP_LOWP_XRUN
-#define MFP_LOWP_XRUN 1
-#endif
-// The 16-bit ELL kernel's VEC path (8 consecutive rows per thread, 16-byte
-// loads) when the layout allows it (1), or always the lane-interleaved path (0).
-#ifndef MFP_LOWP_ELL_VEC
-#define MFP_LOWP_ELL_VEC 1
-#endif
+// 8 rows per thread from 1.75M rows on (16-bit offsets, aligned): banded 2M rows
+// 47.0 us against 48.0 with 2 rows per thread and 4M 89.8 against 90.5, but 1M
+// rows 31.2 against 26.4 (its rows / 8 threads do not fill the chip).  Below
+// 200k rows a row per thread (banded 100k 8.7 us against 10.6).
+constexpr uint32_t kLowpEllVecRows = 1750000, kLowpEllPairRows = 200000;
 int lowp_ell_spmv(int vt, uint32_t rows, uint32_t cols_n, uint32_t width, const uint16_t *q, const float *scale,
                   const uint32_t *cols, const uint16_t *off, const float *x, float *y, void *stream) {
   if (vt != MFP_BF16 && vt != MFP_F16) return fail(MFP_ERROR_INVALID_VALUE, "value type must be BF16 or F16");
   if (rows == 0) return ok();
   if (!scale || !y || (width && (!q || !x || (!cols && !off)))) return fail(MFP_ERROR_INVALID_VALUE, "null device array");
   const bool d16 = cols == nullptr;
-  const bool vec = MFP_LOWP_ELL_VEC && rows % 8 == 0 && aligned16(q) && (d16 ? aligned16(off) : aligned16(cols));
+  const bool vec = d16 && rows >= kLowpEllVecRows && rows % 8 == 0 && aligned16(q) && aligned16(off) && aligned16(x) &&
+                   aligned16(y) && aligned16(scale);
+  const bool pairs = rows >= kLowpEllPairRows && rows % 2 == 0 && (reinterpret_cast<uintptr_t>(cols) & 7u) == 0 &&
+                     ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(off)) & 3u) == 0;
   cudaStream_t s = as_stream(stream);
-  const uint32_t grid = ceil_div(ceil_div(rows, 8), d::kBlock);
-#define MFP_LELL(VT, D16)                                                                         \
-  {                                                                                               \
-    d::lowp_ell_args<VT, D16> A{rows, width, cols_n, q, scale, cols, off, x, y};                  \
-    if (MFP_LOWP_XRUN && vec && D16 && aligned16(x) && aligned16(y) && aligned16(scale))          \
-      d::lowp_ell_kernel<VT, D16, true, true><<<grid, d::kBlock, 0, s>>>(A);                      \
-    else if (vec)                                                                                 \
-      d::lowp_ell_kernel<VT, D16, true><<<grid, d::kBlock, 0, s>>>(A);                            \
-    else                                                                                          \
-      d::lowp_ell_kernel<VT, D16, false><<<grid, d::kBlock, 0, s>>>(A);                           \
+  const auto launch = [&](auto k, const auto &A, uint32_t rows_per_thread) {
+    k<<<ceil_div(ceil_div(rows, rows_per_thread), d::kBlock), d::kBlock, 0, s>>>(A);
+  };
+#define MFP_LELL(VT)                                                                          \
+  if (d16) {                                                                                  \
+    const d::lowp_ell_args<VT, true> A{rows, width, cols_n, q, scale, cols, off, x, y};       \
+    if (vec) launch(d::lowp_ell_kernel<VT>, A, 8u);                                           \
+    else if (pairs) launch(d::lowp_ell_rows_kernel<VT, true, 2, 8>, A, 2u);                   \
+    else launch(d::lowp_ell_rows_kernel<VT, true, 1, 8>, A, 1u);                              \
+  } else {                                                                                    \
+    const d::lowp_ell_args<VT, false> A{rows, width, cols_n, q, scale, cols, off, x, y};      \
+    if (pairs) launch(d::lowp_ell_rows_kernel<VT, false, 2, 8>, A, 2u);                       \
+    else launch(d::lowp_ell_rows_kernel<VT, false, 1, 8>, A, 1u);                             \
   }
   if (vt == MFP_BF16) {
-    if (d16) MFP_LELL(2, true) else MFP_LELL(2, false)
+    MFP_LELL(2)
   } else {
-    if (d16) MFP_LELL(3, true) else MFP_LELL(3, false)
+    MFP_LELL(3)
   }
 #undef MFP_LELL
-  return check_launch("lowp_ell_kernel launch");
+  return check_launch("lowp_ell kernel launch");
 }
 
 // Hybrid: the ELL kernel writes every row's ELL part, then the tile-based COO

@@ -541,17 +541,12 @@ __global__ void __launch_bounds__(kLowpThreads, 3) lowp_tma_kernel(const lowp_ar
 // Reduced-precision ELL: column-major slots [k * rows + row] (the reference's
 // ELL order), 16-bit values q with one FP32 scale per row, and either uint32
 // column ids or 16-bit column offsets from the row (col = row + off - 32768).
-// Padding slots hold q = 0 and a column of their row.  A thread owns 8 rows:
-// VEC (rows % 8 == 0, 16-byte-aligned arrays) 8 consecutive rows, one 16-byte
-// load of 8 values and one of 8 offsets (or two of ids) per slot; otherwise 8
-// rows interleaved across its warp (row = warp base + 32 j + lane), so each
-// 2-byte load and each x gather is contiguous over the warp.  Slots in order
+// Padding slots hold q = 0 and a column of their row.  Slots in order
 // 0..width-1, FMA accumulation; y = acc * scale.
-// With 16-bit offsets, a lane whose 8 rows have the same offset in a slot
-// (stencil rows away from the grid's faces) reads their 8 consecutive x
-// entries with two or three 16-byte loads instead of 8 gathers: a warp's
-// x reads then cover 8 cache lines per instruction instead of 32 sectors,
-// which lifts the L1 limit of the gathers.  Other lanes gather.
+//   lowp_ell_rows_kernel  2 consecutive rows per thread (or 1), 8 slots' loads in
+//                         flight; every layout and alignment
+//   lowp_ell_kernel       8 consecutive rows per thread, one slot in flight; large
+//                         matrices with 16-bit offsets and aligned arrays
 // ---------------------------------------------------------------------------
 template <int VT, bool D16>
 struct lowp_ell_args {
@@ -564,11 +559,9 @@ struct lowp_ell_args {
   float *__restrict__ y;
 };
 
-// CTAs per SM the 16-bit ELL kernel (16-bit offsets, 8 rows per thread) is
-// register-limited to: 8 (32 registers) holds the 27-point 128^3 stencil's
-// 1,024 CTAs in one wave on 148 SMs (6, at 40 registers, left a second wave
-// of 136 CTAs).  The uint32-column variants keep 6 (40 registers, which they
-// need without spilling).
+// CTAs per SM lowp_ell_kernel is register-limited to: 8 (32 registers) holds the
+// 27-point 128^3 stencil's 1,024 CTAs in one wave on 148 SMs (6, at 40
+// registers, left a second wave of 136 CTAs).
 #ifndef MFP_LOWP_ELL_MINBLOCKS
 #define MFP_LOWP_ELL_MINBLOCKS 8
 #endif
@@ -584,108 +577,129 @@ __device__ __forceinline__ void ld_x8_run(const float *__restrict__ x, uint32_t 
   for (int j = 0; j < 8; ++j) xv[j] = sh == 0 ? w[j] : sh == 1 ? w[j + 1] : sh == 2 ? w[j + 2] : w[j + 3];
 }
 
-// XRUN (16-bit offsets, 16-byte-aligned x, y and scale): a thread whose 8
-// rows share one offset in a slot reads their 8 consecutive x entries as
-// three 16-byte loads instead of 8 gathers, and the scales and y move 16
-// bytes at a time.  One slot is in flight, to stay within 32 registers.
-template <int VT, bool D16, bool VEC, bool XRUN = false>
-__global__ void __launch_bounds__(kBlock, D16 && VEC ? MFP_LOWP_ELL_MINBLOCKS : 6)
-    lowp_ell_kernel(const lowp_ell_args<VT, D16> A) {
+// 8 consecutive rows per thread (rows % 8 == 0, 16-byte-aligned arrays): one
+// 16-byte load of 8 values and one of 8 offsets per slot.  A thread whose 8 rows
+// share one offset in a slot (stencil rows away from the grid's faces) reads
+// their 8 consecutive x entries as two or three 16-byte loads instead of 8
+// gathers, and the scales and y move 16 or 32 bytes at a time.  One slot is in
+// flight, to stay within 32 registers.
+template <int VT>
+__global__ void __launch_bounds__(kBlock, MFP_LOWP_ELL_MINBLOCKS) lowp_ell_kernel(const lowp_ell_args<VT, true> A) {
   const uint64_t pol = policy_evict_first();
   const size_t stride = A.n_rows;
-  if (VEC) {
-    const uint32_t r = (blockIdx.x * kBlock + threadIdx.x) * 8u;
-    if (r >= A.n_rows) return;
-    float acc[8];
+  const uint32_t r = (blockIdx.x * kBlock + threadIdx.x) * 8u;
+  if (r >= A.n_rows) return;
+  float acc[8];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) acc[j] = 0.f;
-#pragma unroll(XRUN ? 1 : 2)
-    for (uint32_t k = 0; k < A.width; ++k) {
-      const size_t o = (size_t)k * stride + r;
-      uint32_t qv[4], c[8];
-      ld_stream8_u16(A.q + o, qv, pol);
-      bool run = false;
-      if (D16) {
-        uint32_t dv[4];
-        ld_stream8_u16(A.off + o, dv, pol);
+  for (int j = 0; j < 8; ++j) acc[j] = 0.f;
+#pragma unroll(1)
+  for (uint32_t k = 0; k < A.width; ++k) {
+    const size_t o = (size_t)k * stride + r;
+    uint32_t qv[4], dv[4], c[8];
+    ld_stream8_u16(A.q + o, qv, pol);
+    ld_stream8_u16(A.off + o, dv, pol);
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          c[2 * j] = r + 2u * j + (dv[j] & 0xffffu) - 32768u;
-          c[2 * j + 1] = r + 2u * j + 1u + (dv[j] >> 16) - 32768u;
-        }
-        if (XRUN) {
-          // the 8 rows share one offset: their columns are c[0] .. c[0] + 7
-          const uint32_t d2 = (dv[0] & 0xffffu) | (dv[0] << 16);
-          run = dv[0] == d2 && dv[1] == d2 && dv[2] == d2 && dv[3] == d2 && A.n_cols >= 12u &&
-                c[0] <= A.n_cols - 12u;  // (c[0] & ~3) + 12 <= n_cols, overflow-free
-        }
-      } else {
-        ld_stream8_any(A.cols + o, c, pol);
-      }
-      float xv[8];
-      if (run) {
-        ld_x8_run(A.x, c[0], xv);
-      } else {
-#pragma unroll
-        for (int j = 0; j < 8; ++j) xv[j] = ld_x(A.x + c[j]);
-      }
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const float2 f = lowp_pair<VT>(qv[j]);
-        acc[2 * j] = __fmaf_rn(f.x, xv[2 * j], acc[2 * j]);
-        acc[2 * j + 1] = __fmaf_rn(f.y, xv[2 * j + 1], acc[2 * j + 1]);
-      }
+    for (int j = 0; j < 4; ++j) {
+      c[2 * j] = r + 2u * j + (dv[j] & 0xffffu) - 32768u;
+      c[2 * j + 1] = r + 2u * j + 1u + (dv[j] >> 16) - 32768u;
     }
-    if (XRUN && ((reinterpret_cast<uintptr_t>(A.y) | reinterpret_cast<uintptr_t>(A.scale)) & 31u) == 0) {
-      // 32-byte-aligned y and scale (r is a multiple of 8): one sector each
-      float sc[8];
-      ld_stream8(A.scale + r, sc, pol);
-#pragma unroll
-      for (int j = 0; j < 8; ++j) acc[j] *= sc[j];
-      st_global8(A.y + r, acc);
-    } else if (XRUN) {  // 16-byte-aligned y and scale
-      const float4 s0 = __ldg(reinterpret_cast<const float4 *>(A.scale + r));
-      const float4 s1 = __ldg(reinterpret_cast<const float4 *>(A.scale + r + 4));
-      *reinterpret_cast<float4 *>(A.y + r) = make_float4(acc[0] * s0.x, acc[1] * s0.y, acc[2] * s0.z, acc[3] * s0.w);
-      *reinterpret_cast<float4 *>(A.y + r + 4) =
-          make_float4(acc[4] * s1.x, acc[5] * s1.y, acc[6] * s1.z, acc[7] * s1.w);
+    // the 8 rows share one offset: their columns are c[0] .. c[0] + 7
+    const uint32_t d2 = (dv[0] & 0xffffu) | (dv[0] << 16);
+    const bool run = dv[0] == d2 && dv[1] == d2 && dv[2] == d2 && dv[3] == d2 && A.n_cols >= 12u &&
+                     c[0] <= A.n_cols - 12u;  // (c[0] & ~3) + 12 <= n_cols, overflow-free
+    float xv[8];
+    if (run) {
+      ld_x8_run(A.x, c[0], xv);
     } else {
 #pragma unroll
-      for (int j = 0; j < 8; ++j) A.y[r + j] = acc[j] * A.scale[r + j];
-    }
-  } else {
-    // 8 rows per thread, interleaved across the warp: row = warp base + 32 j +
-    // lane, so every load and every x gather of a warp is contiguous
-    const uint32_t lane = threadIdx.x & 31u;
-    const uint32_t wbase = (blockIdx.x * kBlock + (threadIdx.x & ~31u)) * 8u;
-    if (wbase >= A.n_rows) return;
-    float acc[8];
-    bool ok[8];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      acc[j] = 0.f;
-      ok[j] = wbase + 32u * j + lane < A.n_rows;
-    }
-    for (uint32_t k = 0; k < A.width; ++k) {
-      const size_t o = (size_t)k * stride + wbase + lane;
-      uint32_t qv[8], c[8];
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const uint32_t r = wbase + 32u * j + lane;
-        qv[j] = ok[j] ? ld_stream_u16(A.q + o + 32u * j, pol) : 0u;
-        c[j] = ok[j] ? (D16 ? r + ld_stream_u16(A.off + o + 32u * j, pol) - 32768u : ld_stream1(A.cols + o + 32u * j, pol))
-                     : 0u;
-      }
-      float xv[8];
-#pragma unroll
-      for (int j = 0; j < 8; ++j) xv[j] = ok[j] ? ld_x(A.x + c[j]) : 0.f;
-#pragma unroll
-      for (int j = 0; j < 8; ++j) acc[j] = __fmaf_rn(lowp_to_float<VT>(qv[j]), xv[j], acc[j]);
+      for (int j = 0; j < 8; ++j) xv[j] = ld_x(A.x + c[j]);
     }
 #pragma unroll
-    for (int j = 0; j < 8; ++j)
-      if (ok[j]) A.y[wbase + 32u * j + lane] = acc[j] * A.scale[wbase + 32u * j + lane];
+    for (int j = 0; j < 4; ++j) {
+      const float2 f = lowp_pair<VT>(qv[j]);
+      acc[2 * j] = __fmaf_rn(f.x, xv[2 * j], acc[2 * j]);
+      acc[2 * j + 1] = __fmaf_rn(f.y, xv[2 * j + 1], acc[2 * j + 1]);
+    }
   }
+  if (((reinterpret_cast<uintptr_t>(A.y) | reinterpret_cast<uintptr_t>(A.scale)) & 31u) == 0) {
+    // 32-byte-aligned y and scale (r is a multiple of 8): one sector each
+    float sc[8];
+    ld_stream8(A.scale + r, sc, pol);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) acc[j] *= sc[j];
+    st_global8(A.y + r, acc);
+  } else {  // 16-byte-aligned y and scale
+    const float4 s0 = __ldg(reinterpret_cast<const float4 *>(A.scale + r));
+    const float4 s1 = __ldg(reinterpret_cast<const float4 *>(A.scale + r + 4));
+    *reinterpret_cast<float4 *>(A.y + r) = make_float4(acc[0] * s0.x, acc[1] * s0.y, acc[2] * s0.z, acc[3] * s0.w);
+    *reinterpret_cast<float4 *>(A.y + r + 4) = make_float4(acc[4] * s1.x, acc[5] * s1.y, acc[6] * s1.z, acc[7] * s1.w);
+  }
+}
+
+// R rows per thread (2 consecutive ones, a 4-byte load of values and of offsets
+// per slot, or 1) with U slots' loads in flight.  8 rows per thread with one slot
+// in flight made a small or middle-sized matrix a chain of width load latencies
+// on a few CTAs, and rows not a multiple of 8 were read 2 bytes at a time.  B200,
+// 16-bit offsets: banded 100k rows 27 -> 8.7 us, 300k 27 -> 12.7, 1M 31 -> 26.4,
+// 1,000,001 rows 65 -> 35; 27-point 60^3 31 -> 10.8, 81^3 52 -> 21; uint32 columns,
+// banded 1,000,001 rows 102 -> 38, 2M 89 -> 68.
+template <int VT, bool D16, int R, int U>
+__device__ __forceinline__ void lowp_ell_slots(const lowp_ell_args<VT, D16> &A, uint32_t r, size_t o, float (&acc)[R],
+                                               uint64_t pol) {
+  uint32_t q[U], c[U][R];
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    const size_t i = o + u * (size_t)A.n_rows;
+    if constexpr (R == 2) {
+      q[u] = ld_stream1(reinterpret_cast<const uint32_t *>(A.q + i), pol);
+      if (D16) {
+        const uint32_t w = ld_stream1(reinterpret_cast<const uint32_t *>(A.off + i), pol);
+        c[u][0] = r + (w & 0xffffu) - 32768u;
+        c[u][1] = r + 1u + (w >> 16) - 32768u;
+      } else {
+        ld_stream8_u8(reinterpret_cast<const uint8_t *>(A.cols + i), c[u], pol);  // 8 bytes: two column ids
+      }
+    } else {
+      q[u] = ld_stream_u16(A.q + i, pol);
+      c[u][0] = D16 ? r + ld_stream_u16(A.off + i, pol) - 32768u : ld_stream1(A.cols + i, pol);
+    }
+  }
+  float xv[U][R];
+#pragma unroll
+  for (int u = 0; u < U; ++u)
+#pragma unroll
+    for (int j = 0; j < R; ++j) xv[u][j] = ld_x(A.x + c[u][j]);
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    if constexpr (R == 2) {
+      const float2 f = lowp_pair<VT>(q[u]);
+      acc[0] = __fmaf_rn(f.x, xv[u][0], acc[0]);
+      acc[1] = __fmaf_rn(f.y, xv[u][1], acc[1]);
+    } else {
+      acc[0] = __fmaf_rn(lowp_to_float<VT>(q[u]), xv[u][0], acc[0]);
+    }
+  }
+}
+template <int VT, bool D16, int R, int U>
+__global__ void __launch_bounds__(kBlock) lowp_ell_rows_kernel(const lowp_ell_args<VT, D16> A) {
+  const uint64_t pol = policy_evict_first();
+  const uint32_t r = (blockIdx.x * kBlock + threadIdx.x) * R;
+  if (r >= A.n_rows) return;
+  float sc[R], acc[R];
+#pragma unroll
+  for (int j = 0; j < R; ++j) {
+    sc[j] = __ldg(A.scale + r + j);
+    acc[j] = 0.f;
+  }
+  uint32_t k = 0;
+  for (; k + U <= A.width; k += U) lowp_ell_slots<VT, D16, R, U>(A, r, (size_t)k * A.n_rows + r, acc, pol);
+  if (U > 4 && k + 4u <= A.width) {
+    lowp_ell_slots<VT, D16, R, 4>(A, r, (size_t)k * A.n_rows + r, acc, pol);
+    k += 4u;
+  }
+  for (; k < A.width; ++k) lowp_ell_slots<VT, D16, R, 1>(A, r, (size_t)k * A.n_rows + r, acc, pol);
+#pragma unroll
+  for (int j = 0; j < R; ++j) A.y[r + j] = acc[j] * sc[j];
 }
 
 }  // namespace dev

@@ -214,3 +214,42 @@ def test_ell_widths_and_row_counts(width, rows, dtype):
         s = slice(k * rows, (k + 1) * rows)
         want = want + e.data[s] * x[e.columns[s]]
     assert np.array_equal(y.view(np.uint8), want.astype(dtype).view(np.uint8))
+
+
+@pytest.mark.parametrize("rows, width", [(1, 3), (199_999, 9), (200_000, 8), (200_002, 7), (200_001, 12), (1_750_000, 5),
+                                         (1_750_004, 4)])
+@pytest.mark.parametrize("index16", [False, True])
+@pytest.mark.parametrize("vt", [2, 3])
+def test_lowp_ell_rows_per_thread(rows, width, index16, vt):
+    """16-bit ELL on both sides of the row counts where a thread takes 1, 2 or 8
+    rows, at widths around the slots in flight: the same bits whether the
+    arrays' alignment lets a thread take several rows or not, and y within FP32
+    rounding of the 64-bit product."""
+    rng = np.random.default_rng(rows + width)
+    cols = rows + 500
+    n = rows * width
+    off = rng.integers(-200, 200, n)
+    off[rng.random(n) < 0.5] = 3  # runs of equal offsets
+    row = np.tile(np.arange(rows), width)
+    col = np.clip(row + off, 0, cols - 1)
+    bits = torch.from_numpy(rng.uniform(-1, 1, n).astype(np.float32)).to(torch.bfloat16 if vt == 2 else torch.float16)
+    scale = rng.uniform(0.5, 2, rows).astype(np.float32)
+    x = rng.uniform(-1, 1, cols).astype(np.float32)
+    idx = (col - row + 32768).astype(np.uint16) if index16 else col.astype(np.uint32)
+    outs = []
+    for shift in (0, 1):  # elements past an aligned start
+        q = torch.zeros(n + 8, dtype=torch.int16, device="cuda")
+        q[shift:shift + n] = bits.view(torch.int16).cuda()
+        ix = torch.zeros(n + 8, dtype=torch.int16 if index16 else torch.int32, device="cuda")
+        ix[shift:shift + n] = dev(idx.view(np.int16 if index16 else np.int32))
+        sc, xt = dev(scale), dev(x)
+        y = torch.full((rows,), float("nan"), device="cuda")
+        call("mfp_lowp_ell_spmv", vt, rows, cols, width, p(q[shift:]), p(sc), None if index16 else p(ix[shift:]),
+             p(ix[shift:]) if index16 else None, p(xt), p(y), None)
+        torch.cuda.synchronize()
+        outs.append(y.cpu().numpy())
+    assert np.array_equal(outs[0].view(np.uint32), outs[1].view(np.uint32))
+    prod = bits.double().numpy() * x[col].astype(np.float64)
+    want = prod.reshape(width, rows).sum(0) * scale
+    bound = (width + 1) * 2.0 ** -23 * np.abs(prod).reshape(width, rows).sum(0) * scale
+    assert np.all(np.abs(outs[0] - want) <= bound + 1e-30)
