@@ -248,6 +248,20 @@ constexpr uint32_t kDefaultAssist = 64;
 // with 8 lanes (128 bytes) ran 378 us on 8M rows and with 4 lanes 485, which
 // fetch a line's halves at different times; in FP64 (4M rows) 4 lanes ran 274 us
 // and 8 lanes 298.  *regular = elements in blocks without either.
+// (row_blocks_regular: the share of that from every n-th block, to tell a
+// power-law matrix without reading all of its row_ptr.)
+bool row_blocks_regular(uint32_t rows, const uint32_t *rp) {
+  const uint32_t n = ceil_div(rows, d::kBlock), step = std::max(1u, n / 512u);
+  uint64_t seen = 0, regular = 0;
+  for (uint32_t b = 0; b < n; b += step) {
+    const uint32_t r0 = b * d::kBlock, r1 = std::min(rows, r0 + d::kBlock);
+    bool all_short = true;
+    for (uint32_t r = r0; r < r1 && all_short; ++r) all_short = rp[r + 1] - rp[r] <= kDefaultAssist;
+    seen += rp[r1] - rp[r0];
+    regular += all_short ? rp[r1] - rp[r0] : 0u;
+  }
+  return 5 * regular >= 2 * seen;  // 40%: the plan asks for half of all
+}
 std::vector<uint4> row_block_info(uint32_t rows, const uint32_t *rp, uint32_t long_thr, uint32_t assist_thr,
                                   uint64_t *regular) {
   std::vector<uint4> br(ceil_div(rows, d::kBlock));
@@ -426,7 +440,7 @@ extern "C" int mfp_csr_plan_create(uint32_t rows, uint32_t cols, uint32_t nnz, c
   // matrix has a row above 64 elements in nine blocks of ten and keeps its
   // kernels.
   std::vector<uint4> blk;
-  if (MFP_CSR_DIRECT && automatic && nnz) {
+  if (MFP_CSR_DIRECT && automatic && nnz && row_blocks_regular(rows, rp)) {
     uint64_t regular = 0;
     blk = row_block_info(rows, rp, kDefaultLong, kDefaultAssist, &regular);
     plan->direct = 16 * regular >= 15ull * nnz || (2 * regular >= nnz && nnz >= kDirectMixed);
@@ -542,16 +556,15 @@ extern "C" int mfp_csr_plan_create(uint32_t rows, uint32_t cols, uint32_t nnz, c
       if (bins && !left_out(blocks[b])) continue;
       const uint32_t r0 = bins ? blocks[b] : b * d::kBlock;
       const uint32_t r1 = bins ? blocks[b + 1] : std::min(rows, r0 + d::kBlock);
-      uint64_t c = r1 - r0;
-      for (uint32_t r = r0; r < r1; ++r) {
-        const uint32_t len = rp[r + 1] - rp[r];
-        if (len <= cfg.long_row_threshold) c += len;
-      }
-      cost[b] = c;
+      cost[b] = (uint64_t)(r1 - r0) + (rp[r1] - rp[r0]);  // less its long rows, below
       order.push_back(b);
     }
     for (uint32_t k = 0; k < plan->n_pieces; ++k) {
-      cost[plan->n_main + k] = pieces[k].e1 - pieces[k].e0;
+      const d::long_piece &pc = pieces[k];
+      const uint32_t b = bins ? (uint32_t)(std::upper_bound(blocks.begin(), blocks.end(), pc.row) - blocks.begin()) - 1u
+                              : pc.row / d::kBlock;
+      cost[b] -= pc.e1 - pc.e0;
+      cost[plan->n_main + k] = pc.e1 - pc.e0;
       order.push_back(plan->n_main + k);
     }
     std::stable_sort(order.begin(), order.end(), [&](uint32_t a, uint32_t b) { return cost[a] > cost[b]; });
@@ -755,11 +768,15 @@ int csr_spmv(const mfp_csr_plan *plan, const T *data, const uint32_t *cols, cons
     if (rest && !seq) { MFP_CSR_LAUNCH_N(2, false, rest) }
     if (vec) {
       auto k = seq ? d::csr_direct_kernel<T, true> : d::csr_direct_kernel<T, false>;
+      // few row blocks: several CTAs each, until the chip's 148 x 8 are in use
+      const uint32_t n_blk = ceil_div(plan->rows, d::kBlock);
+      uint32_t split = 1;
+      while (split < 16u && n_blk * split * 2u <= 148u * 8u) split *= 2;
       if (rest) {  // beside the blocks with longer rows
-        const cudaError_t e = launch_after(k, ceil_div(plan->rows, d::kBlock), s, A);
+        const cudaError_t e = launch_after(k, n_blk * split, s, A, split);
         if (e != cudaSuccess) return cuda_fail(e, "csr_direct_kernel launch");
       } else {
-        k<<<ceil_div(plan->rows, d::kBlock), d::kBlock, 0, s>>>(A);
+        k<<<n_blk * split, d::kBlock, 0, s>>>(A, split);
       }
     }
     return check_launch("csr_direct_kernel launch");
@@ -1562,13 +1579,14 @@ int scoo_attach_windows(mfp_matrix *m, const std::vector<uint32_t> &win, const u
 //  - when the heaviest slice holds more than twice the mean, which that
 //    slice's CTA would work through alone (B200: power-law, 50k rows FP32 49.7
 //    -> 13.7 us, 1M rows FP64 107 -> 59 us, 4M rows FP32 184 -> 170 us);
-//  - when there is work for the whole chip, and the slices are fewer than the
-//    148 x 6 CTAs it holds or so short (under 16 tiles) that their CTA's
+//  - when there is work for the whole chip, and the slices are fewer than four
+//    per SM or so short (under 16 tiles) that their CTA's
 //    rounds of 8 tiles, barriers and x window weigh (27-point 40^3, 148
 //    slices, FP32 17.8 -> 12.1 us; 5-point 1400^2 FP64, 10 tiles each, 79.8 ->
 //    49.9 us; 1000^2 FP32 27.2 -> 22.6 us).
 // Long balanced slices stay with the one launch (27-point 128^3 122 us against
-// 139, banded 2M rows 118 against 128: no tile table to wait for), and so do
+// 139, banded 2M rows 118 against 128, 400k rows 28.5 against 31.4: no tile table
+// to wait for), and so do
 // small matrices, where the second launch costs more than it gives (64 x 64
 // Laplacian 8.4 us against 11.1).
 bool scoo_use_tiles(const mfp_matrix *m, const uint32_t *sp_host) {
@@ -1578,7 +1596,7 @@ bool scoo_use_tiles(const mfp_matrix *m, const uint32_t *sp_host) {
     if (sp_host[s + 1] > sp_host[s]) heaviest = std::max<uint64_t>(heaviest, sp_host[s + 1] - sp_host[s]);
   const uint64_t mean = m->nnz / std::max<uint64_t>(1, used);
   if (heaviest > 2 * mean && heaviest > 16 * d::kWarpTile) return true;
-  return (used < 148u * 6u || mean < 16 * d::kWarpTile) && m->nnz >= 148u * 6u * d::kWarpTile * 4u;
+  return (used < 148u * 4u || mean < 16 * d::kWarpTile) && m->nnz >= 148u * 6u * d::kWarpTile * 4u;
 }
 
 // Row-ordered SCOO: every slice's 256-element tiles (an entry without elements
