@@ -236,7 +236,9 @@ int mfp_dev_scratch_release(void);
 typedef enum mfp_csr_algo { MFP_CSR_SCALAR = 0, MFP_CSR_VECTOR = 1, MFP_CSR_ADAPTIVE = 2 } mfp_csr_algo;
 typedef struct mfp_csr_config {
   uint32_t long_row_threshold; /* 0 = default for the algo; UINT32_MAX = never split */
-  uint32_t vector_lanes;       /* CSR vector lanes per row: 2..32 (power of two); 0 = auto:
+  uint32_t vector_lanes;       /* CSR vector lanes per row: 2..32 (power of two); 0 = auto: blocks
+                                  of short rows straight from global memory when they hold most
+                                  elements; else
                                   below a mean row length of 64 the warp-tile kernel (each
                                   warp's lanes take 8 consecutive elements of 256 and combine
                                   rows with a segmented shuffle scan; a fix-up launch adds the

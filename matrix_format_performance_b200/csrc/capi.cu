@@ -2515,7 +2515,8 @@ int mfp_batch_get_info(const mfp_batch *b, mfp_batch_info *out) {
   out->algorithmic_bytes = b->algorithmic_bytes;
   out->device_bytes = b->array_bytes + (b->plan ? b->plan->device_bytes : 0);
   out->config = b->cfg;
-  out->kernel_launches = b->nnz ? 1 : (b->rows ? 1 : 0);
+  out->kernel_launches = b->rows ? 1u : 0u;
+  if (b->nnz && (b->plan->tile || (b->plan->direct && b->plan->n_order))) out->kernel_launches = 2u;
   return ok();
 }
 
@@ -2539,7 +2540,8 @@ int mfp_batch_spmv(const mfp_batch *b, const void *x, void *y, void *stream) {
 int mfp_batch_autotune(mfp_batch *b, const void *x, void *y, uint32_t reps, void *stream, mfp_batch_config *chosen,
                        double *best_seconds) {
   if (!b || reps == 0) return fail(MFP_ERROR_INVALID_VALUE, "bad argument");
-  // the candidate plans: CSR scalar with several warp-assist and long-row
+  // the candidate plans: each algorithm's automatic plan (short rows straight
+  // from global memory), CSR scalar with several warp-assist and long-row
   // thresholds, the streaming (persistent) kernel, CSR vector lane counts and
   // CSR-Adaptive bin sizes
   std::vector<mfp_batch_config> cand;
@@ -2553,6 +2555,7 @@ int mfp_batch_autotune(mfp_batch *b, const void *x, void *y, uint32_t reps, void
     c.csr.kernel = kernel;
     cand.push_back(c);
   };
+  for (int algo : {0, 1, 2}) add(algo, 0, 0, 0, 0, 0);
   for (uint32_t assist : {32u, 64u, 256u})
     for (uint32_t longt : {2048u, 4096u, 16384u}) add(0, 0, 0, assist, longt, 1);
   add(0, 0, 0, 0, 0, 2);
