@@ -225,7 +225,11 @@ int mfp_dev_scratch_release(void);
 /* ------------------------------------------------------------------------- */
 
 /* CSR family.  A plan partitions the rows once per sparsity pattern (long-row
- * pieces, CSR-Adaptive row bins) and owns the scratch the pieces combine in.
+ * pieces, CSR-Adaptive row bins).  The scratch that a row's pieces combine in
+ * is each call's own, so calls on one plan may overlap on several streams; the
+ * streaming and warp-tile kernels (configuration kernel 2 to 4, and CSR vector
+ * without a configuration on matrices of mixed rows) keep theirs in the plan,
+ * and their calls must not overlap.
  * algo: 0 = CSR scalar (one thread per row; csr_spmv_kernel,
  * gpu_matrix_multiplier.cu:22-43), 1 = CSR vector (a lane group per row;
  * csr_spmv_vector_kernel, :331-362), 2 = CSR-Adaptive (row bins;

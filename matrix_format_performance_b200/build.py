@@ -27,8 +27,9 @@ NVCC = str(CUDA_HOME / "bin" / "nvcc")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 
 CU_SOURCES = ["capi.cu", "convert.cu"]
-CPP_SOURCES = ["util.cpp", "formats.cpp", "synth.cpp"]
-HEADERS = ["spmv_device.cuh", "spmv_kernels.cuh", "spmv_stream.cuh", "spmv_lowp.cuh", "mlp.cuh", "host_common.h"]
+CPP_SOURCES = ["util.cpp", "scratch.cpp", "formats.cpp", "synth.cpp"]
+HEADERS = ["spmv_device.cuh", "spmv_kernels.cuh", "spmv_stream.cuh", "spmv_lowp.cuh", "mlp.cuh", "host_common.h",
+           "scratch.h"]
 
 NVCC_FLAGS = ARCH + ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-Xptxas", "-O3",
                      "--expt-relaxed-constexpr", f"-I{ROOT / 'include'}"]

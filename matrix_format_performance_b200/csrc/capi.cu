@@ -1,5 +1,6 @@
 // C ABI: plans, kernel launches, device-resident matrix handles and timing.
 #include "host_common.h"
+#include "scratch.h"
 #include "spmv_kernels.cuh"
 #include "spmv_stream.cuh"
 #include "spmv_lowp.cuh"
@@ -184,8 +185,10 @@ struct mfp_csr_plan {
   uint32_t rows = 0, cols = 0, nnz = 0;
   uint32_t n_main = 0, n_pieces = 0, n_long = 0;
   d::long_piece *pieces = nullptr;
-  double *partials = nullptr;
-  uint32_t *counters = nullptr;
+  // a call's scratch for the rows of several pieces: an arrival counter per row
+  // (n_counters, zero between calls), then (piece_partials) the pieces' sums
+  call_blocks piece_ws;
+  uint32_t n_counters = 0;
   uint32_t *row_blocks = nullptr;
   uint32_t *order = nullptr;  // work items heaviest first
   uint32_t n_order = 0;       // n_main + n_pieces; direct plans: the items left to csr_kernel
@@ -293,6 +296,8 @@ std::vector<uint4> row_block_info(uint32_t rows, const uint32_t *rp, uint32_t lo
 // us, 300k rows FP32 31.5 -> 17.9, 1M rows FP64 74 -> 50, 4M rows unchanged;
 // nnz / 1024 and nnz / 4096 were 0-4 us slower from 300k rows on.
 constexpr uint32_t kDefaultPiece = 65536, kMinPiece = 2048, kPieceShare = 512;
+// Bytes of the counters at the head of a call's long-row scratch.
+size_t piece_partials(uint32_t n_counters) { return ((size_t)n_counters * sizeof(uint32_t) + 15u) & ~(size_t)15u; }
 constexpr uint32_t kFp64Rows = 4096;  // rows longer than this accumulate in FP64
 constexpr uint32_t kMaxBin = d::kChunk - 4;
 }  // namespace
@@ -498,11 +503,14 @@ extern "C" int mfp_csr_plan_create(uint32_t rows, uint32_t cols, uint32_t nnz, c
       pc.slot_base = slots;
       pc.piece = k;
       pc.npieces = np;
-      pc.counter = nlong;
+      pc.counter = plan->n_counters;
       pc.fp64 = len > kFp64Rows ? 1u : 0u;
       pieces.push_back(pc);
     }
-    if (np > 1) slots += np;
+    if (np > 1) {
+      slots += np;
+      ++plan->n_counters;
+    }
     ++nlong;
   }
   std::vector<uint32_t> blocks;
@@ -572,8 +580,6 @@ extern "C" int mfp_csr_plan_create(uint32_t rows, uint32_t cols, uint32_t nnz, c
   plan->n_order = (uint32_t)order.size();
   if ((st = upload(&plan->order, order.data(), order.size(), &plan->device_bytes)) ||
       (st = upload(&plan->pieces, pieces.data(), pieces.size(), &plan->device_bytes)) ||
-      (st = dmalloc(&plan->partials, slots, &plan->device_bytes)) ||
-      (st = dmalloc(&plan->counters, nlong, &plan->device_bytes)) ||
       (st = upload(&plan->row_blocks, blocks.data(), blocks.size(), &plan->device_bytes))) {
     mfp_csr_plan_destroy(plan);
     return st;
@@ -607,11 +613,13 @@ extern "C" int mfp_csr_plan_create(uint32_t rows, uint32_t cols, uint32_t nnz, c
     }
     plan->tile_ws = ws;
   }
-  if (nlong) {
-    const cudaError_t e = cudaMemset(plan->counters, 0, nlong * sizeof(uint32_t));
+  if (slots) {
+    const size_t counters = piece_partials(plan->n_counters);
+    const cudaError_t e = plan->piece_ws.init(counters + slots * sizeof(double), counters, &plan->device_bytes);
     if (e != cudaSuccess) {
       mfp_csr_plan_destroy(plan);
-      return cuda_fail(e, "cudaMemset counters");
+      return fail(e == cudaErrorMemoryAllocation ? MFP_ERROR_OUT_OF_MEMORY : MFP_ERROR_CUDA, "long-row scratch: %s",
+                  cudaGetErrorString(e));
     }
   }
   *out = plan;
@@ -621,8 +629,6 @@ extern "C" int mfp_csr_plan_create(uint32_t rows, uint32_t cols, uint32_t nnz, c
 extern "C" int mfp_csr_plan_destroy(mfp_csr_plan *plan) {
   if (!plan) return ok();
   cudaFree(plan->pieces);
-  cudaFree(plan->partials);
-  cudaFree(plan->counters);
   cudaFree(plan->row_blocks);
   cudaFree(plan->order);
   cudaFree(plan->error);
@@ -713,8 +719,6 @@ int csr_spmv(const mfp_csr_plan *plan, const T *data, const uint32_t *cols, cons
   A.n_main = plan->n_main;
   A.n_pieces = plan->n_pieces;
   A.pieces = plan->pieces;
-  A.partials = plan->partials;
-  A.counters = plan->counters;
   A.order = MFP_CSR_ORDER ? plan->order : nullptr;
   A.blk = plan->blk;
   const bool vec = aligned16(data) && aligned16(cols);
@@ -753,6 +757,11 @@ int csr_spmv(const mfp_csr_plan *plan, const T *data, const uint32_t *cols, cons
   if (plan->tile && !exact_order) return csr_tile_spmv<T>(plan, data, cols, rp, x, y, s);
   const uint32_t grid = plan->n_main + plan->n_pieces;
   if (grid == 0) return ok();
+  const call_scratch ws(plan->piece_ws, s);
+  if (ws.ptr()) {  // NULL: no row of several pieces, or no memory
+    A.counters = static_cast<uint32_t *>(ws.ptr());
+    A.partials = reinterpret_cast<double *>(static_cast<unsigned char *>(ws.ptr()) + piece_partials(plan->n_counters));
+  }
 #define MFP_CSR_LAUNCH_N(ALGO, FAST, N)                                              \
   if (vec)                                                                           \
     d::csr_kernel<T, ALGO, true, FAST><<<N, d::kBlock, 0, s>>>(A);                   \
@@ -977,20 +986,20 @@ int scoo_spmv(uint32_t rows, uint32_t slices, uint32_t slice, const T *v, const 
 // the handle, given back with it), so calls on different streams never share
 // it; under stream capture it becomes an allocation of the graph.  p stays
 // NULL when there is no memory.
-struct call_scratch {
+struct pool_scratch {
   cudaStream_t s;
   void *p = nullptr;
-  call_scratch(cudaMemPool_t pool, size_t bytes, cudaStream_t st) : s(st) {
+  pool_scratch(cudaMemPool_t pool, size_t bytes, cudaStream_t st) : s(st) {
     if (pool && bytes && cudaMallocFromPoolAsync(&p, bytes, pool, st) != cudaSuccess) {
       cudaGetLastError();
       p = nullptr;
     }
   }
-  ~call_scratch() {
+  ~pool_scratch() {
     if (p) cudaFreeAsync(p, s);
   }
-  call_scratch(const call_scratch &) = delete;
-  call_scratch &operator=(const call_scratch &) = delete;
+  pool_scratch(const pool_scratch &) = delete;
+  pool_scratch &operator=(const pool_scratch &) = delete;
 };
 
 // A pool whose freed memory stays mapped for the next call; `bytes`, one
@@ -1003,7 +1012,7 @@ int make_call_pool(int device, size_t bytes, cudaMemPool_t *pool) {
   CUDA_TRY(cudaMemPoolCreate(pool, &props), "cudaMemPoolCreate");
   uint64_t keep = UINT64_MAX;
   CUDA_TRY(cudaMemPoolSetAttribute(*pool, cudaMemPoolAttrReleaseThreshold, &keep), "cudaMemPoolSetAttribute");
-  { const call_scratch warm(*pool, bytes, nullptr); }
+  { const pool_scratch warm(*pool, bytes, nullptr); }
   CUDA_TRY(cudaStreamSynchronize(nullptr), "cudaStreamSynchronize");
   return MFP_SUCCESS;
 }
@@ -1405,7 +1414,7 @@ struct mfp_matrix {
   uint32_t *tile_base = nullptr;
   uint8_t *rel8 = nullptr;  // COO / hybrid tail: 8-bit offsets (tiles of at most 256 rows)
   uint32_t wide_tiles = 0;  // with rel8: tiles spanning more rows, which read rows_a / rows2
-  cudaMemPool_t pool = nullptr;       // call scratch (see call_scratch)
+  cudaMemPool_t pool = nullptr;       // call scratch (see pool_scratch)
   void *dx = nullptr, *dy = nullptr;  // staging for the host-buffer call
   // second staging pair, copy streams and events of the pipelined host-buffer
   // call (made on its first use)
@@ -2124,7 +2133,7 @@ int mfp_matrix_spmv(const mfp_matrix *m, const void *x, void *y, void *stream) {
                                             m->rows_a, m->aux, m->win, m->max_window, m->order, (const float *)x,
                                             (float *)y, stream);
       if (m->tiles) {
-        const call_scratch ws(m->pool, m->ws_bytes, as_stream(stream));
+        const pool_scratch ws(m->pool, m->ws_bytes, as_stream(stream));
         if (ws.p)  // without memory for the carries: one CTA per slice
           return f64 ? scoo_tile_spmv<double>(m->rows, m->slice_size, m->n_tiles, m->tiles, (const double *)m->vals,
                                               m->cols_a, m->rows_a, m->rel, (const double *)x, (double *)y, ws.p, stream)

@@ -692,8 +692,8 @@ struct csr_args {
   uint32_t n_main;
   uint32_t n_pieces;
   const long_piece *__restrict__ pieces;
-  double *partials;
-  uint32_t *counters;
+  double *partials;    // the call's scratch for rows of several pieces (NULL: none)
+  uint32_t *counters;  // zero before and after the call
   // work item of each block index (w < n_main: row block / bin w, else piece
   // w - n_main), heaviest first; NULL = blocks in index order
   const uint32_t *__restrict__ order;
@@ -995,7 +995,12 @@ __global__ void __launch_bounds__(kBlock, sizeof(T) == 4 ? (ALGO != 1 ? MFP_CSR_
   else
     w = blockIdx.x;
   if (w >= A.n_main) {
-    const long_piece pc = A.pieces[w - A.n_main];
+    long_piece pc = A.pieces[w - A.n_main];
+    if (pc.npieces > 1 && !A.counters) {  // no scratch to combine in: one CTA takes the whole row
+      if (pc.piece) return;
+      pc.e1 = A.row_ptr[pc.row + 1];
+      pc.npieces = 1;
+    }
     run_piece<T, VEC>(pc, A.vals, A.cols, A.x, A.y, A.partials, A.counters, sm.p.a, sm.p.b, pol);
     return;
   }
