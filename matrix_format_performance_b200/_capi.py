@@ -223,6 +223,7 @@ _PROTOS.update({
     "mfp_scoo_spmv_unsorted_f32": [u32, u32, u32, u32, vp, vp, vp, vp, vp, u32, vp, vp, vp, vp],
     "mfp_scoo_spmv_unsorted_f64": [u32, u32, u32, u32, vp, vp, vp, vp, vp, u32, vp, vp, vp, vp],
     "mfp_dev_csr_from_coo": [i32, u32, u32, u32, vp, vp, vp, vp, vp, vp, vp],
+    "mfp_dev_csr_from_coo_limited": [i32, u32, u32, u32, vp, vp, vp, vp, vp, vp, u32, vp],
     "mfp_dev_scratch_bytes": [C.POINTER(u64)],
     "mfp_dev_scratch_release": [],
     "mfp_matrix_create_device": [i32, i32, u32, u32, u32, vp, vp, vp, C.POINTER(DeviceBuildOptions),

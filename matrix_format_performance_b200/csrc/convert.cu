@@ -40,6 +40,7 @@ constexpr uint32_t kRadixBins = 1u << kRadixBits;
 static_assert(kRadixBins == kRadixThreads, "one thread per digit");
 constexpr uint32_t kRadixPasses = 8;                      // 64-bit keys
 constexpr uint32_t kRadixPolls = 1u << 20;                // look-back limit, about a second
+constexpr uint32_t kNoTile = 0xffffffffu;
 
 int cuda_fail(cudaError_t e, const char *what) {
   return fail(MFP_ERROR_CUDA, "%s: %s", what, cudaGetErrorString(e));
@@ -668,6 +669,11 @@ __device__ __forceinline__ unsigned long long ld_status(const unsigned long long
   asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
   return v;
 }
+__device__ __forceinline__ uint32_t ld_word(const uint32_t *p) {
+  uint32_t v;
+  asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
 __device__ __forceinline__ void st_status(unsigned long long *p, unsigned long long v) {
   asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
@@ -680,7 +686,9 @@ __device__ __forceinline__ void st_status(unsigned long long *p, unsigned long l
 // is placed in shared memory in digit order and written out as contiguous digit
 // runs; payloads follow through the same shared memory.  Tiles are numbered in
 // the order their CTAs start, so a tile only ever waits for CTAs that are
-// running; the wait is bounded (err[3]).
+// running.  The wait is bounded: a tile that gives up after `polls` looks sets
+// err[3] and scatters nothing (without its count its keys could land anywhere),
+// and what is launched or starts after that returns at once.
 struct radix_smem {
   unsigned long long key[kRadixTile];  // or payloads
   uint32_t wh[kRadixWarps][kRadixBins];
@@ -691,17 +699,22 @@ struct radix_smem {
 template <uint32_t BITS, typename P, typename In, typename Out>
 __global__ void __launch_bounds__(kRadixThreads, 2) radix_pass_kernel(uint32_t n, In in, Out out, uint32_t pass,
                                                                       const uint32_t *hist, uint32_t *counter,
-                                                                      unsigned long long *status, uint32_t *err) {
+                                                                      unsigned long long *status, uint32_t polls,
+                                                                      uint32_t *err) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   radix_smem &S = *reinterpret_cast<radix_smem *>(smem_raw);
   constexpr uint32_t kPerWarp = kRadixTile / kRadixWarps;
   const uint32_t t = threadIdx.x, lane = t & 31u, warp = t >> 5;
-  if (t == 0) S.tile = atomicAdd(counter, 1u);
+  if (t == 0) {
+    const uint32_t gave_up = ld_word(err + 3), at = atomicAdd(counter, 1u);
+    S.tile = gave_up ? kNoTile : at;
+  }
 #pragma unroll
   for (uint32_t i = 0; i < kRadixWarps; ++i) S.wh[i][t] = 0u;
   const uint32_t hv = hist[t];
   __syncthreads();
   const uint32_t tile = S.tile, shift = pass * BITS;
+  if (tile == kNoTile) return;
   const uint64_t base = (uint64_t)tile * kRadixTile;
   const uint32_t tn = (uint32_t)min((uint64_t)kRadixTile, n - base);
   const uint32_t wbase = warp * kPerWarp + lane;
@@ -754,26 +767,27 @@ __global__ void __launch_bounds__(kRadixThreads, 2) radix_pass_kernel(uint32_t n
     }
   // the same digit's keys in earlier tiles
   uint32_t excl = 0;
-  if (tile) {
+  bool found = tile == 0;
+  if (!found) {
     const unsigned long long *st = status + t;
-    for (uint32_t w = tile - 1u, polls = 0;;) {
+    for (uint32_t w = tile - 1u; polls;) {
       const unsigned long long v = ld_status(st + (size_t)w * kRadixBins);
       const uint32_t flag = (uint32_t)(v >> 32);
       if (flag <= 2u * pass) {  // not there yet
-        if (++polls > kRadixPolls) {
-          atomicOr(&err[3], 1u);
-          break;
-        }
+        --polls;
         continue;
       }
       excl += (uint32_t)v;
-      if (flag == 2u * pass + 2u || w == 0) break;
+      if ((found = flag == 2u * pass + 2u || w == 0)) break;
       --w;
     }
-    st_status(mine, status_word(pass, true, excl + tot));
+    if (found) st_status(mine, status_word(pass, true, excl + tot));
   }
   S.gbase[t] = below + excl - start;
-  __syncthreads();
+  if (__syncthreads_or(!found)) {
+    if (t == 0) atomicOr(&err[3], 1u);
+    return;
+  }
   uint32_t g[kRadixRounds];
 #pragma unroll
   for (uint32_t j = 0; j < kRadixRounds; ++j) {
@@ -800,11 +814,13 @@ __global__ void __launch_bounds__(kRadixThreads, 2) radix_pass_kernel(uint32_t n
 }
 
 // row_ptr from sorted rows: position p starts the rows (rows[p-1], rows[p]]
-// (p = nnz closes the rows after the last element's row).
+// (p = nnz closes the rows after the last element's row).  Nothing after a sort
+// that gave up, whose rows are not ids.
 __global__ void __launch_bounds__(kThreads) rowptr_from_rows_kernel(uint32_t nnz, uint32_t rows,
-                                                                    const uint32_t *__restrict__ ri, uint32_t *rp) {
+                                                                    const uint32_t *__restrict__ ri, uint32_t *rp,
+                                                                    const uint32_t *err) {
   const uint64_t p = (uint64_t)blockIdx.x * kThreads + threadIdx.x;
-  if (p > nnz) return;
+  if (p > nnz || __ldg(err + 3)) return;
   const uint32_t cur = p < nnz ? ri[p] : rows;
   for (uint32_t q = p ? ri[p - 1] + 1u : 0u; q <= cur; ++q) rp[q] = (uint32_t)p;
 }
@@ -878,12 +894,12 @@ struct radix_state {
 };
 template <typename P, typename In, typename Out>
 int radix_pass(uint32_t n, const In &in, const Out &out, const radix_digits &dg, uint32_t pass, const radix_state &R,
-               uint32_t *err, scratch &sc) {
+               uint32_t polls, uint32_t *err, scratch &sc) {
   auto k = dg.bits == 8u ? radix_pass_kernel<8, P, In, Out> : radix_pass_kernel<9, P, In, Out>;
   CV_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(radix_smem)),
          "cudaFuncSetAttribute");
   k<<<R.tiles, kRadixThreads, sizeof(radix_smem), sc.st>>>(n, in, out, pass, R.hist + pass * kRadixBins,
-                                                           R.counters + pass, R.status, err);
+                                                           R.counters + pass, R.status, polls, err);
   CV_TRY(cudaGetLastError(), "radix_pass_kernel");
   return MFP_SUCCESS;
 }
@@ -909,7 +925,7 @@ int radix_sort_pairs(uint32_t n, uint32_t bits, unsigned long long *&k0, P *&p0,
                                                                                  dg.passes, R.hist, err);
   CV_TRY(cudaGetLastError(), "radix_hist_kernel");
   for (uint32_t pass = 0; pass < dg.passes; ++pass) {
-    if ((s = radix_pass<P>(n, pairs_in<P>{k0, p0}, pairs_out<P>{k1, p1}, dg, pass, R, err, sc))) return s;
+    if ((s = radix_pass<P>(n, pairs_in<P>{k0, p0}, pairs_out<P>{k1, p1}, dg, pass, R, kRadixPolls, err, sc))) return s;
     std::swap(k0, k1);
     std::swap(p0, p1);
   }
@@ -920,7 +936,7 @@ int radix_sort_pairs(uint32_t n, uint32_t bits, unsigned long long *&k0, P *&p0,
 
 template <typename T>
 int csr_from_coo_t(uint32_t rows, uint32_t cols, uint32_t nnz, const uint32_t *ri, const uint32_t *ci,
-                   const double *v, uint32_t *rp, uint32_t *co, T *data, void *stream) {
+                   const double *v, uint32_t *rp, uint32_t *co, T *data, uint32_t polls, void *stream) {
   cudaStream_t st = as_stream(stream);
   scratch sc(st);
   if (!rp) return fail(MFP_ERROR_INVALID_VALUE, "null row_ptr");
@@ -966,15 +982,16 @@ int csr_from_coo_t(uint32_t rows, uint32_t cols, uint32_t nnz, const uint32_t *r
       const pairs_in<T> mid_in{k[(pass + 1u) & 1u], p[(pass + 1u) & 1u]};
       const pairs_out<T> mid_out{k[pass & 1u], p[pass & 1u]};
       if (first)
-        s = last ? radix_pass<T>(nnz, in, out, dg, pass, R, err, sc) : radix_pass<T>(nnz, in, mid_out, dg, pass, R, err, sc);
+        s = last ? radix_pass<T>(nnz, in, out, dg, pass, R, polls, err, sc)
+                 : radix_pass<T>(nnz, in, mid_out, dg, pass, R, polls, err, sc);
       else
-        s = last ? radix_pass<T>(nnz, mid_in, out, dg, pass, R, err, sc)
-                 : radix_pass<T>(nnz, mid_in, mid_out, dg, pass, R, err, sc);
+        s = last ? radix_pass<T>(nnz, mid_in, out, dg, pass, R, polls, err, sc)
+                 : radix_pass<T>(nnz, mid_in, mid_out, dg, pass, R, polls, err, sc);
       if (s) return s;
     }
     sorted_rows = out_rows;
   }
-  rowptr_from_rows_kernel<<<blocks_for((uint64_t)nnz + 1, kThreads), kThreads, 0, st>>>(nnz, rows, sorted_rows, rp);
+  rowptr_from_rows_kernel<<<blocks_for((uint64_t)nnz + 1, kThreads), kThreads, 0, st>>>(nnz, rows, sorted_rows, rp, err);
   CV_TRY(cudaGetLastError(), "rowptr_from_rows_kernel");
   CV_TRY(cudaMemcpyAsync(h_err, err, sizeof(h_err), cudaMemcpyDeviceToHost, st), "cudaMemcpyAsync");
   CV_TRY(cudaStreamSynchronize(st), "cudaStreamSynchronize");
@@ -1214,10 +1231,16 @@ int mfp_dev_scratch_bytes(uint64_t *reserved) {
 
 int mfp_dev_csr_from_coo(int vt, uint32_t rows, uint32_t cols, uint32_t nnz, const uint32_t *ri, const uint32_t *ci,
                          const double *v, uint32_t *rp, uint32_t *co, void *data, void *stream) {
+  return mfp_dev_csr_from_coo_limited(vt, rows, cols, nnz, ri, ci, v, rp, co, data, kRadixPolls, stream);
+}
+
+int mfp_dev_csr_from_coo_limited(int vt, uint32_t rows, uint32_t cols, uint32_t nnz, const uint32_t *ri,
+                                 const uint32_t *ci, const double *v, uint32_t *rp, uint32_t *co, void *data,
+                                 uint32_t polls, void *stream) {
   if (!valid_vt(vt)) return fail(MFP_ERROR_INVALID_VALUE, "bad value type");
   if (vt == MFP_F64)
-    return csr_from_coo_t<double>(rows, cols, nnz, ri, ci, v, rp, co, static_cast<double *>(data), stream);
-  return csr_from_coo_t<float>(rows, cols, nnz, ri, ci, v, rp, co, static_cast<float *>(data), stream);
+    return csr_from_coo_t<double>(rows, cols, nnz, ri, ci, v, rp, co, static_cast<double *>(data), polls, stream);
+  return csr_from_coo_t<float>(rows, cols, nnz, ri, ci, v, rp, co, static_cast<float *>(data), polls, stream);
 }
 
 }  // extern "C"
