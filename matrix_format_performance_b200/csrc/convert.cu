@@ -14,6 +14,7 @@
 //     tiles rank their keys, look back for the counts of the tiles before them
 //     and scatter) for COO triplets -> CSR on the composite key (row, column).
 #include "host_common.h"
+#include "row_span.h"
 
 #include <cuda_runtime.h>
 
@@ -821,8 +822,8 @@ __global__ void __launch_bounds__(kThreads) rowptr_from_rows_kernel(uint32_t nnz
                                                                     const uint32_t *err) {
   const uint64_t p = (uint64_t)blockIdx.x * kThreads + threadIdx.x;
   if (p > nnz || __ldg(err + 3)) return;
-  const uint32_t cur = p < nnz ? ri[p] : rows;
-  for (uint32_t q = p ? ri[p - 1] + 1u : 0u; q <= cur; ++q) rp[q] = (uint32_t)p;
+  const row_span span = rows_starting_at(p, nnz, p ? ri[p - 1] : 0u, p < nnz ? ri[p] : 0u, rows);
+  for (uint64_t q = span.first; q < span.end; ++q) rp[q] = (uint32_t)p;
 }
 
 // Triplets already in CSR order.
