@@ -209,7 +209,8 @@ int mfp_dev_scoo_x_windows(uint32_t nnz, const uint32_t *c_index, const uint32_t
  * from device COO triplets in any order (waits): row_ptr by histogram and
  * scan, elements ordered by (row, column) with a stable radix sort, so
  * repeated (row, column) entries keep their input order like
- * mfp_csr_from_coo.  Out-of-range ids return MFP_ERROR_INVALID_VALUE. */
+ * mfp_csr_from_coo.  Out-of-range ids return MFP_ERROR_INVALID_VALUE.  The
+ * outputs may be the inputs' memory (columns = col_ids, data = values). */
 int mfp_dev_csr_from_coo(int value_type, uint32_t rows, uint32_t cols, uint32_t nnz, const uint32_t *row_ids,
                          const uint32_t *col_ids, const double *values, uint32_t *row_ptr, uint32_t *columns,
                          void *data, void *stream);

@@ -935,6 +935,27 @@ int radix_sort_pairs(uint32_t n, uint32_t bits, unsigned long long *&k0, P *&p0,
   return radix_error(h_err[3]);
 }
 
+struct byte_range {
+  const void *p;
+  size_t bytes;
+  bool overlaps(const byte_range &o) const {
+    const uintptr_t a = reinterpret_cast<uintptr_t>(p), b = reinterpret_cast<uintptr_t>(o.p);
+    return a < b + o.bytes && b < a + bytes;
+  }
+};
+// An input that an output overlaps moves to scratch.
+template <typename I>
+int unshare(const I *&in, size_t n, const byte_range (&outs)[3], scratch &sc) {
+  const byte_range r{in, n * sizeof(I)};
+  if (!r.overlaps(outs[0]) && !r.overlaps(outs[1]) && !r.overlaps(outs[2])) return MFP_SUCCESS;
+  I *copy = nullptr;
+  const int s = sc.get(&copy, n);
+  if (s) return s;
+  CV_TRY(cudaMemcpyAsync(copy, in, r.bytes, cudaMemcpyDeviceToDevice, sc.st), "cudaMemcpyAsync");
+  in = copy;
+  return MFP_SUCCESS;
+}
+
 template <typename T>
 int csr_from_coo_t(uint32_t rows, uint32_t cols, uint32_t nnz, const uint32_t *ri, const uint32_t *ci,
                    const double *v, uint32_t *rp, uint32_t *co, T *data, uint32_t polls, void *stream) {
@@ -955,16 +976,22 @@ int csr_from_coo_t(uint32_t rows, uint32_t cols, uint32_t nnz, const uint32_t *r
   if ((s = sc.get(&err, 4)) || (s = R.begin(nnz, dg, sc))) return s;
   const uint32_t err_init[4] = {0u, 0xffffffffu, 0u, 0u};
   CV_TRY(cudaMemcpyAsync(err, err_init, sizeof(err_init), cudaMemcpyHostToDevice, st), "cudaMemcpyAsync");
-  const triplets_in<T> in{ri, ci, v, cb};
   auto hk = dg.bits == 8u ? radix_hist_kernel<true, 8, triplets_in<T>> : radix_hist_kernel<true, 9, triplets_in<T>>;
-  hk<<<std::min(kKeyBlocks, blocks_for(nnz, 4u * kThreads)), kThreads, 0, st>>>(nnz, in, rows, cols, dg.passes, R.hist,
-                                                                                err);
+  hk<<<std::min(kKeyBlocks, blocks_for(nnz, 4u * kThreads)), kThreads, 0, st>>>(nnz, triplets_in<T>{ri, ci, v, cb}, rows,
+                                                                                cols, dg.passes, R.hist, err);
   CV_TRY(cudaGetLastError(), "radix_hist_kernel");
   uint32_t h_err[4];
   CV_TRY(cudaMemcpyAsync(h_err, err, sizeof(h_err), cudaMemcpyDeviceToHost, st), "cudaMemcpyAsync");
   CV_TRY(cudaStreamSynchronize(st), "cudaStreamSynchronize");
   if (h_err[0] & 1u) return fail(MFP_ERROR_INVALID_VALUE, "row id >= rows %u at element %u", rows, h_err[1]);
   if (h_err[0] & 2u) return fail(MFP_ERROR_INVALID_VALUE, "col id >= cols %u at element %u", cols, h_err[1]);
+  // a kernel that reads the triplets and writes the CSR needs them apart (several
+  // passes read them all into scratch first)
+  if (!h_err[2] || dg.passes == 1u) {
+    const byte_range outs[3] = {{rp, ((size_t)rows + 1) * 4u}, {co, (size_t)nnz * 4u}, {data, (size_t)nnz * sizeof(T)}};
+    if ((s = unshare(ri, nnz, outs, sc)) || (s = unshare(ci, nnz, outs, sc)) || (s = unshare(v, nnz, outs, sc))) return s;
+  }
+  const triplets_in<T> in{ri, ci, v, cb};
   const uint32_t *sorted_rows = ri;
   if (!h_err[2]) {  // in CSR order already: a stable sort would keep it
     csr_copy_kernel<T><<<blocks_for(nnz, kThreads), kThreads, 0, st>>>(nnz, ci, v, co, data);

@@ -1,4 +1,5 @@
-"""Edges of the device triplets -> CSR conversion: waits that run out."""
+"""Edges of the device triplets -> CSR conversion: waits that run out,
+outputs in the inputs' memory."""
 import ctypes as C
 
 import numpy as np
@@ -66,3 +67,23 @@ def test_one_tile_never_waits():
     order = np.lexsort((np.arange(TILE), c, r))
     assert np.array_equal(outs[1].cpu().numpy(), c[order])
     assert np.array_equal(outs[2].cpu().numpy(), v[order])
+
+
+@pytest.mark.parametrize("order", ["sorted", "shuffled"])
+@pytest.mark.parametrize("rows, cols", [(3, 200), (70_000, 65_537)])  # one digit (one pass), four digits
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+def test_outputs_in_the_inputs_memory(order, rows, cols, dtype):
+    """columns = col_ids, data = values and row_ptr = row_ids give what separate
+    outputs give."""
+    n = 100 * TILE + 5
+    r, c, v = triplets(rows, cols, n, seed=9)
+    if order == "sorted":
+        k = np.lexsort((c, r))
+        r, c, v = r[k], c[k], v[k]
+    want = [t.cpu().numpy() for t in convert.csr_from_coo(rows, cols, dev(r), dev(c), dev(v), dtype=dtype)]
+    tr, tc, tv = dev(r), dev(c), dev(v)
+    call("mfp_dev_csr_from_coo", int(dtype == torch.float64), rows, cols, n, p(tr), p(tc), p(tv), p(tr), p(tc), p(tv),
+         None)
+    got = tr[:rows + 1], tc, tv.view(dtype)[:n]
+    for g, w in zip(got, want):
+        assert np.array_equal(g.cpu().numpy(), w)
