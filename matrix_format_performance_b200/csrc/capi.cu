@@ -981,42 +981,6 @@ int scoo_spmv(uint32_t rows, uint32_t slices, uint32_t slice, const T *v, const 
   return scoo_launch<T, 0, false>(slices, dyn, s, rows, slice, v, ci, ri, sp, win, maxw, order, x, y);
 }
 
-// Scratch of one SpMV call on a handle that several streams may use at once:
-// allocated and freed in stream order from the handle's own pool (made with
-// the handle, given back with it), so calls on different streams never share
-// it; under stream capture it becomes an allocation of the graph.  p stays
-// NULL when there is no memory.
-struct pool_scratch {
-  cudaStream_t s;
-  void *p = nullptr;
-  pool_scratch(cudaMemPool_t pool, size_t bytes, cudaStream_t st) : s(st) {
-    if (pool && bytes && cudaMallocFromPoolAsync(&p, bytes, pool, st) != cudaSuccess) {
-      cudaGetLastError();
-      p = nullptr;
-    }
-  }
-  ~pool_scratch() {
-    if (p) cudaFreeAsync(p, s);
-  }
-  pool_scratch(const pool_scratch &) = delete;
-  pool_scratch &operator=(const pool_scratch &) = delete;
-};
-
-// A pool whose freed memory stays mapped for the next call; `bytes`, one
-// call's scratch, are mapped here rather than by the first call.
-int make_call_pool(int device, size_t bytes, cudaMemPool_t *pool) {
-  cudaMemPoolProps props{};
-  props.allocType = cudaMemAllocationTypePinned;
-  props.location.type = cudaMemLocationTypeDevice;
-  props.location.id = device;
-  CUDA_TRY(cudaMemPoolCreate(pool, &props), "cudaMemPoolCreate");
-  uint64_t keep = UINT64_MAX;
-  CUDA_TRY(cudaMemPoolSetAttribute(*pool, cudaMemPoolAttrReleaseThreshold, &keep), "cudaMemPoolSetAttribute");
-  { const pool_scratch warm(*pool, bytes, nullptr); }
-  CUDA_TRY(cudaStreamSynchronize(nullptr), "cudaStreamSynchronize");
-  return MFP_SUCCESS;
-}
-
 // Row-ordered SCOO handles: the slices' warp tiles, then the fix-up.
 template <typename T>
 int scoo_tile_spmv(uint32_t rows, uint32_t slice, uint32_t n_tiles, const d::scoo_tile *tiles, const T *v,
@@ -1414,7 +1378,6 @@ struct mfp_matrix {
   uint32_t *tile_base = nullptr;
   uint8_t *rel8 = nullptr;  // COO / hybrid tail: 8-bit offsets (tiles of at most 256 rows)
   uint32_t wide_tiles = 0;  // with rel8: tiles spanning more rows, which read rows_a / rows2
-  cudaMemPool_t pool = nullptr;       // call scratch (see pool_scratch)
   void *dx = nullptr, *dy = nullptr;  // staging for the host-buffer call
   // second staging pair, copy streams and events of the pipelined host-buffer
   // call (made on its first use)
@@ -1426,7 +1389,8 @@ struct mfp_matrix {
   uint16_t *delta = nullptr;          // 16-bit column deltas (else cols_a)
   uint32_t *base = nullptr;
   bool rows_unsorted = false;         // SCOO in the sort_cols layout
-  d::scoo_tile *tiles = nullptr;      // row-ordered SCOO: the slices' warp tiles (carries: ws_bytes of call scratch)
+  d::scoo_tile *tiles = nullptr;      // row-ordered SCOO: the slices' warp tiles
+  call_blocks carry_ws;               // their carries, per call
   uint32_t n_tiles = 0;
   bool long_rows = false;             // reduced-precision CSR: a row longer than kLowpTmaMaxRow
 };
@@ -1609,7 +1573,7 @@ bool scoo_use_tiles(const mfp_matrix *m, const uint32_t *sp_host) {
 }
 
 // Row-ordered SCOO: every slice's 256-element tiles (an entry without elements
-// for an empty slice, whose rows it zeroes) and the workspace of their carries.
+// for an empty slice, whose rows it zeroes) and the scratch of their carries.
 int scoo_attach_tiles(mfp_matrix *m, const uint32_t *sp_host) {
   std::vector<d::scoo_tile> t;
   t.reserve((size_t)m->nnz / d::kWarpTile + m->slices);
@@ -1627,9 +1591,11 @@ int scoo_attach_tiles(mfp_matrix *m, const uint32_t *sp_host) {
     }
   }
   m->n_tiles = (uint32_t)t.size();
-  m->ws_bytes = carry_ws_bytes(m->n_tiles);
-  const int st = make_call_pool(m->device, m->ws_bytes, &m->pool);
-  return st ? st : track_upload(m, &m->tiles, t.data(), t.size());
+  const cudaError_t e = m->carry_ws.init(carry_ws_bytes(m->n_tiles), 0, &m->device_bytes);
+  if (e != cudaSuccess)
+    return fail(e == cudaErrorMemoryAllocation ? MFP_ERROR_OUT_OF_MEMORY : MFP_ERROR_CUDA, "SCOO carries: %s",
+                cudaGetErrorString(e));
+  return track_upload(m, &m->tiles, t.data(), t.size());
 }
 
 int check_columns(const uint32_t *c, uint64_t n, uint32_t cols) {
@@ -1652,7 +1618,6 @@ int mfp_matrix_destroy(mfp_matrix *m) {
   if (m->s_in) cudaStreamDestroy(m->s_in);
   if (m->s_out) cudaStreamDestroy(m->s_out);
   for (void *p : m->allocs) cudaFree(p);
-  if (m->pool) cudaMemPoolDestroy(m->pool);
   mfp_csr_plan_destroy(m->plan);
   delete m;
   return ok();
@@ -2133,12 +2098,13 @@ int mfp_matrix_spmv(const mfp_matrix *m, const void *x, void *y, void *stream) {
                                             m->rows_a, m->aux, m->win, m->max_window, m->order, (const float *)x,
                                             (float *)y, stream);
       if (m->tiles) {
-        const pool_scratch ws(m->pool, m->ws_bytes, as_stream(stream));
-        if (ws.p)  // without memory for the carries: one CTA per slice
+        const call_scratch ws(m->carry_ws, as_stream(stream));
+        if (ws.ptr())  // without memory for the carries: one CTA per slice
           return f64 ? scoo_tile_spmv<double>(m->rows, m->slice_size, m->n_tiles, m->tiles, (const double *)m->vals,
-                                              m->cols_a, m->rows_a, m->rel, (const double *)x, (double *)y, ws.p, stream)
+                                              m->cols_a, m->rows_a, m->rel, (const double *)x, (double *)y, ws.ptr(),
+                                              stream)
                      : scoo_tile_spmv<float>(m->rows, m->slice_size, m->n_tiles, m->tiles, (const float *)m->vals,
-                                             m->cols_a, m->rows_a, m->rel, (const float *)x, (float *)y, ws.p, stream);
+                                             m->cols_a, m->rows_a, m->rel, (const float *)x, (float *)y, ws.ptr(), stream);
       }
       return f64 ? scoo_spmv<double>(m->rows, m->slices, m->slice_size, (const double *)m->vals, m->cols_a,
                                      m->rows_a, m->aux, m->win, m->max_window, m->order, (const double *)x,

@@ -1,6 +1,7 @@
 """One handle, plan or batch used by several streams, threads and captured graphs
 at once: each call's scratch is its own, so every result has the bits of a lone
 call."""
+import ctypes as C
 import threading
 
 import numpy as np
@@ -11,8 +12,11 @@ pytestmark = pytest.mark.gpu
 
 from matrix_format_performance_b200 import formats as F  # noqa: E402
 from matrix_format_performance_b200 import synth  # noqa: E402
+from matrix_format_performance_b200._capi import call  # noqa: E402
 from matrix_format_performance_b200.batch import Batch  # noqa: E402
-from matrix_format_performance_b200.device import CSR_ADAPTIVE, CSR_SCALAR, DeviceMatrix  # noqa: E402
+from matrix_format_performance_b200.device import CSR_ADAPTIVE, CSR_SCALAR, SCOO, DeviceMatrix  # noqa: E402
+
+TOL = {np.float32: 1e-5, np.float64: 1e-12}  # per row, of sum |a_ij x_j|
 
 
 def long_rows(dtype, rows=3000, cols=70_000, seed=31):
@@ -106,12 +110,22 @@ def test_batch_rows_of_several_pieces():
     b.close()
 
 
-def test_captured_calls_allocate_nothing_in_the_graph():
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+def test_scoo_tiles(dtype):
+    m = long_rows(dtype)
+    dm = DeviceMatrix.build(m, SCOO)
+    assert dm.info().kernel_launches == 2  # tiles and fix-up
+    check_all(lambda x, y, s: dm.spmv(x, y, s), vectors(m, 3), m.rows)
+    dm.close()
+
+
+@pytest.mark.parametrize("fmt", [CSR_ADAPTIVE, SCOO])
+def test_captured_calls_allocate_nothing_in_the_graph(fmt):
     """A captured call is kernel launches only, so its graph can be cloned, be a
     child graph and be instantiated again."""
     rt = pytest.importorskip("cuda.bindings.runtime")
     m = long_rows(np.float32)
-    dm = DeviceMatrix.from_csr(m, CSR_ADAPTIVE)
+    dm = DeviceMatrix.build(m, fmt)
     x = vectors(m, 1)[0]
     y, want = (torch.empty(m.rows, device="cuda") for _ in range(2))
     dm.spmv(x, want)
@@ -128,4 +142,57 @@ def test_captured_calls_allocate_nothing_in_the_graph():
     torch.cuda.synchronize()
     assert same(y, want)
     del g
+    dm.close()
+
+
+@pytest.fixture
+def no_device_memory():
+    """take(stream): allocates all device memory that is left."""
+    rt = pytest.importorskip("cuda.bindings.runtime")
+    held = []
+
+    def take(stream):
+        torch.cuda.empty_cache()
+        size = 1 << 36
+        while size >= 1 << 20:
+            err, p = rt.cudaMalloc(size)
+            if int(err):
+                rt.cudaGetLastError()
+                size >>= 1
+            else:
+                held.append(p)
+        assert int(rt.cudaMallocAsync(1, stream.cuda_stream)[0])
+        rt.cudaGetLastError()
+
+    yield take
+    for p in held:
+        rt.cudaFree(p)
+
+
+@pytest.mark.parametrize("fmt", [CSR_ADAPTIVE, CSR_SCALAR, SCOO])
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+def test_calls_without_memory_for_their_scratch(oracle_lib, no_device_memory, fmt, dtype):
+    """With no memory left, a second stream's call runs without
+    scratch: SCOO one CTA per slice, CSR one CTA per long row."""
+    m = long_rows(dtype)
+    dm = DeviceMatrix.build(m, fmt)
+    x = vectors(m, 1)[0]
+    first, second = (torch.full((m.rows,), float("nan"), dtype=x.dtype, device="cuda") for _ in range(2))
+    if fmt == SCOO:  # its kernel is loaded while there is memory
+        s = F.scoo_matrix_class(148, 49152, m)
+        keep = [torch.from_numpy(np.ascontiguousarray(a)).cuda() for a in
+                (s.values, s.c_index.view(np.int32), s.r_index.view(np.int32), s.slices_ptr.view(np.int32))]
+        v, ci, ri, sp, xp, yp = (C.c_void_p(t.data_ptr()) for t in (*keep, x, first))
+        call(f"mfp_scoo_spmv_{'f32' if dtype == np.float32 else 'f64'}", m.rows, m.cols, s.slices_count, s.slice_size, v,
+             ci, ri, sp, None, 0, None, xp, yp, None)
+        torch.cuda.synchronize()
+    one, two = torch.cuda.Stream(), torch.cuda.Stream()
+    dm.spmv(x, first, one)  # its stream takes the handle's own block
+    torch.cuda.synchronize()
+    no_device_memory(two)
+    dm.spmv(x, second, two)
+    torch.cuda.synchronize()
+    ys, ab = oracle_lib.csr_spmv_exact(m.rows, m.row_ptr, m.columns, m.data, x.cpu().numpy())
+    for y in (first, second):
+        assert np.all(np.abs(y.cpu().numpy().astype(np.float64) - ys) <= TOL[dtype] * ab)
     dm.close()
