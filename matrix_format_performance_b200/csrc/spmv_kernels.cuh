@@ -1242,10 +1242,12 @@ struct coo_carry {
   uint32_t *flags, *tail_row;
 };
 
-// Row ids at or above n_rows (invalid input) are dropped, never written.
-template <typename T, bool ACCUM>
+// Row ids at or above n_rows (invalid input) are dropped, never written.  SLICE:
+// the row's sum starts from +0, as in a slice's zeroed accumulator (a row of -0
+// products is +0).
+template <typename T, bool ACCUM, bool SLICE = false>
 __device__ __forceinline__ void coo_put(T *y, uint32_t n_rows, uint32_t row, T v) {
-  if (row < n_rows) y[row] = ACCUM ? add_rn(y[row], v) : v;
+  if (row < n_rows) y[row] = ACCUM ? add_rn(y[row], v) : SLICE ? add_rn(T(0), v) : v;
 }
 
 // The reduction of one warp tile ending at c1 (of nnz elements), lane l's
@@ -1311,7 +1313,7 @@ __device__ __forceinline__ void warp_tile_reduce(uint32_t wt, uint32_t g0, uint3
           acc = add_rn(acc, pr[k]);
         } else {
           if (first) sf = acc;
-          else coo_put<T, ACCUM>(y, n_rows, cur, acc);
+          else coo_put<T, ACCUM, SLICE>(y, n_rows, cur, acc);
           if (!ACCUM)
             for (uint32_t r = cur + 1u; r < rw[k] && r < n_rows; ++r) y[r] = T(0);
           first = false;
@@ -1371,14 +1373,14 @@ __device__ __forceinline__ void warp_tile_reduce(uint32_t wt, uint32_t g0, uint3
   if (!single) {
     // first run ends inside the lane
     if (from_prev) cw.head[wt] = ftot;
-    else coo_put<T, ACCUM>(y, n_rows, rf, ftot);
+    else coo_put<T, ACCUM, SLICE>(y, n_rows, rf, ftot);
   }
   // last run (the first run too when single)
   const T ltot = single ? ftot : sl;
   const bool l_from_prev = single && from_prev;
   if (after != rl) {
     if (l_from_prev) cw.head[wt] = ltot;
-    else coo_put<T, ACCUM>(y, n_rows, rl, ltot);
+    else coo_put<T, ACCUM, SLICE>(y, n_rows, rl, ltot);
   } else if (lane == last_lane) {
     // the tail row continues into the next tile
     cw.tail[wt] = ltot;

@@ -1,0 +1,58 @@
+"""SCOO handles whose slices run as warp tiles, against one CTA per slice."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+from matrix_format_performance_b200 import formats as F  # noqa: E402
+from matrix_format_performance_b200._capi import call  # noqa: E402
+from matrix_format_performance_b200.device import SCOO, DeviceMatrix  # noqa: E402
+
+
+def dev(a):
+    return torch.from_numpy(np.ascontiguousarray(a)).cuda()
+
+
+def raw_scoo(s, m, x):
+    """y from the raw entry point, which keeps one CTA per slice."""
+    keep = [dev(a) for a in (s.values, s.c_index.view(np.int32), s.r_index.view(np.int32), s.slices_ptr.view(np.int32), x)]
+    y = torch.full((m.rows,), float("nan"), dtype=keep[0].dtype, device="cuda")
+    v, ci, ri, sp, xt = (C.c_void_p(t.data_ptr()) for t in keep)
+    call(f"mfp_scoo_spmv_{'f32' if m.dtype == np.float32 else 'f64'}", m.rows, m.cols, s.slices_count, s.slice_size, v, ci,
+         ri, sp, None, 0, None, xt, C.c_void_p(y.data_ptr()), None)
+    torch.cuda.synchronize()
+    return y.cpu().numpy()
+
+
+def handle_spmv(dm, m, x):
+    xt, y = dev(x), torch.full((m.rows,), float("nan"), dtype=dev(x).dtype, device="cuda")
+    dm.spmv(xt, y)
+    torch.cuda.synchronize()
+    return y.cpu().numpy()
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+def test_rows_of_negative_zero_products(dtype):
+    """Rows whose products are all -0 (one, several, a whole tile and more of
+    them) have the sign that one CTA per slice gives them."""
+    rng = np.random.default_rng(12)
+    lens = rng.integers(0, 9, 3000)
+    lens[700] = 20_000  # uneven slices: the handle runs tiles
+    lens[[40, 1400, 2999]] = 300, 700, 1
+    lens[[10, 11, 12]] = 1, 2, 8
+    rp = np.concatenate([[0], np.cumsum(lens)]).astype(np.uint32)
+    n, cols = int(rp[-1]), 500
+    v = rng.uniform(0.5, 1, n)
+    row = np.repeat(np.arange(3000), lens)
+    zero_rows = np.isin(row, [10, 11, 12, 40, 1400, 2999]) | (row % 5 == 0)
+    v[zero_rows] = -0.0
+    m = F.csr_matrix_class.from_arrays(3000, cols, rp, rng.integers(0, cols, n).astype(np.uint32), v, dtype)
+    x = rng.uniform(0.5, 1, cols).astype(dtype)
+    dm = DeviceMatrix.build(m, SCOO)
+    assert dm.info().kernel_launches == 2  # tiles and fix-up
+    y = handle_spmv(dm, m, x)
+    dm.close()
+    assert np.array_equal(y.view(np.uint8), raw_scoo(F.scoo_matrix_class(148, 49152, m), m, x).view(np.uint8))
