@@ -918,6 +918,16 @@ int csr_tile_spmv(const mfp_csr_plan *plan, const T *data, const uint32_t *cols,
   return ok();
 }
 
+// Shared memory of a slice's CTA: its rows' accumulators and x window.
+template <typename T>
+size_t scoo_dyn_bytes(uint32_t slice, uint32_t window) {
+  return (((size_t)slice + 3u) & ~(size_t)3u) * sizeof(T) + (size_t)window * sizeof(T);
+}
+template <typename T>
+bool scoo_fits(uint32_t slice, uint32_t window) {
+  return scoo_dyn_bytes<T>(slice, window) + sizeof(d::scoo_smem_static<T>) <= 227 * 1024;
+}
+
 template <typename T, int VEC, bool XWIN, bool UNSORTED = false, bool R16 = false>
 int scoo_launch(uint32_t grid, size_t dyn, cudaStream_t s, uint32_t rows, uint32_t slice, const T *v,
                 const uint32_t *ci, const uint32_t *ri, const uint32_t *sp, const uint32_t *win, uint32_t maxw,
@@ -951,10 +961,9 @@ int scoo_spmv(uint32_t rows, uint32_t slices, uint32_t slice, const T *v, const 
   // values / c_index / r_index may be NULL only when every slice is empty
   if (!y || !sp || !x) return fail(MFP_ERROR_INVALID_VALUE, "null device array");
   if (slice == 0 || (uint64_t)slice * slices < rows) return fail(MFP_ERROR_INVALID_VALUE, "slices do not cover the rows");
-  const size_t acc_bytes = (size_t)((slice + 3u) & ~3u) * sizeof(T);
   if (win == nullptr) maxw = 0;
-  const size_t dyn = acc_bytes + (size_t)maxw * sizeof(T);
-  if (dyn + sizeof(d::scoo_smem_static<T>) > 227 * 1024)
+  const size_t dyn = scoo_dyn_bytes<T>(slice, maxw);
+  if (!scoo_fits<T>(slice, maxw))
     return fail(MFP_ERROR_NOT_SUPPORTED, "slice_size %u / window %u too large for shared memory", slice, maxw);
   const int vec = vec_level(v, ci, ri);
   cudaStream_t s = as_stream(stream);
@@ -1562,8 +1571,12 @@ int scoo_attach_windows(mfp_matrix *m, const std::vector<uint32_t> &win, const u
 // to wait for), and so do
 // small matrices, where the second launch costs more than it gives (64 x 64
 // Laplacian 8.4 us against 11.1).
+// Slices whose rows scoo_kernel cannot hold in shared memory stay with it too,
+// and are refused: it is what a call without memory for its carries runs.
 bool scoo_use_tiles(const mfp_matrix *m, const uint32_t *sp_host) {
   if (m->rows_unsorted || m->nnz == 0) return false;
+  const bool f64 = m->value_type == MFP_F64;
+  if (!(f64 ? scoo_fits<double>(m->slice_size, 0) : scoo_fits<float>(m->slice_size, 0))) return false;
   uint64_t heaviest = 0, used = 0;
   for (uint32_t s = 0; s < m->slices && (uint64_t)s * m->slice_size < m->rows; ++s, ++used)
     if (sp_host[s + 1] > sp_host[s]) heaviest = std::max<uint64_t>(heaviest, sp_host[s + 1] - sp_host[s]);

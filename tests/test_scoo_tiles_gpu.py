@@ -8,7 +8,7 @@ torch = pytest.importorskip("torch")
 pytestmark = pytest.mark.gpu
 
 from matrix_format_performance_b200 import formats as F  # noqa: E402
-from matrix_format_performance_b200._capi import call  # noqa: E402
+from matrix_format_performance_b200._capi import MfpError, ScooParams, call  # noqa: E402
 from matrix_format_performance_b200.device import SCOO, DeviceMatrix  # noqa: E402
 
 
@@ -56,3 +56,22 @@ def test_rows_of_negative_zero_products(dtype):
     y = handle_spmv(dm, m, x)
     dm.close()
     assert np.array_equal(y.view(np.uint8), raw_scoo(F.scoo_matrix_class(148, 49152, m), m, x).view(np.uint8))
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+def test_slices_beyond_shared_memory_are_refused(dtype):
+    """A slice whose rows do not fit one CTA's shared memory is refused, whether or
+    not its handle could run warp tiles."""
+    rng = np.random.default_rng(4)
+    rows = 60_000
+    lens = rng.integers(0, 40, rows)
+    rp = np.concatenate([[0], np.cumsum(lens)]).astype(np.uint32)
+    m = F.csr_matrix_class.from_arrays(rows, 100, rp, rng.integers(0, 100, int(rp[-1])).astype(np.uint32),
+                                       rng.uniform(-1, 1, int(rp[-1])), dtype)
+    prm = ScooParams()
+    prm.slices_count, prm.slice_size, prm.lane_size = 1, rows, 1
+    dm = DeviceMatrix.from_device_csr(dev(m.row_ptr.view(np.int32)), dev(m.columns.view(np.int32)), dev(m.data), 100, SCOO,
+                                      scoo=prm)
+    with pytest.raises(MfpError, match="too large for shared memory"):
+        handle_spmv(dm, m, np.ones(100, dtype))
+    dm.close()
