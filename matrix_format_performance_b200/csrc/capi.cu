@@ -198,6 +198,7 @@ struct mfp_csr_plan {
   bool fast = false;     // row blocks without long rows start their loads before the row_ptr barrier
   bool binned = false;   // CSR scalar on the CSR-Adaptive bins, one thread per row
   bool direct = false;   // rows straight from global memory (csr_direct_kernel)
+  bool wide_rows[2] = {false, false};  // most of its elements in blocks of 4 lanes per row or more (FP32, FP64)
   bool tile = false;
   uint32_t *tile_prev = nullptr;
   void *tile_ws = nullptr;
@@ -449,7 +450,14 @@ extern "C" int mfp_csr_plan_create(uint32_t rows, uint32_t cols, uint32_t nnz, c
     uint64_t regular = 0;
     blk = row_block_info(rows, rp, kDefaultLong, kDefaultAssist, &regular);
     plan->direct = 16 * regular >= 15ull * nnz || (2 * regular >= nnz && nnz >= kDirectMixed);
-    if (plan->direct) plan->binned = false;
+    if (plan->direct) {
+      plan->binned = false;
+      uint64_t wide[2] = {0, 0};
+      for (const uint4 &b : blk)
+        for (int t = 0; t < 2; ++t)
+          if (!(b.z & 3u) && ((b.z >> (8 + 8 * t)) & 0xffu) >= 4u) wide[t] += b.y - b.x;
+      for (int t = 0; t < 2; ++t) plan->wide_rows[t] = 2 * wide[t] >= regular;
+    }
   }
   if (algo == MFP_CSR_ADAPTIVE || plan->binned || plan->direct)
     cfg.bin_nnz = cfg.bin_nnz ? std::min(cfg.bin_nnz, kMaxBin) : kMaxBin;
@@ -698,6 +706,23 @@ cudaError_t launch_after(void (*k)(KArgs...), uint32_t grid, cudaStream_t s, Arg
   return cudaLaunchKernelEx(&cfg, k, std::forward<Args>(args)...);
 }
 
+// CTAs per row block of csr_direct_kernel, `wave` of which fit the chip at once.
+// Few blocks: as many as still fit (FP64 100k rows of 4 to 64 elements, 391
+// blocks: 28.1 us with 1, 25.0 with 2, 25.4 with 4; 150k rows, 586 blocks: 32.7
+// with 1, 39.9 with 2, which leave a third of a second wave).  Up to three waves
+// whose last is at most 0.6 full: two CTAs per block, which end it in half the
+// time (344k rows of 4 to 64 elements FP32 64.7 -> 55.7 us, FP64 74.9 -> 69.7;
+// 250k FP64 68.1 -> 55.8; with a fuller last wave, FP64 band 400k rows, 30.7 ->
+// 32.6, and beyond three waves, FP32 27-point 100^3, 50.0 -> 51.9).  Two lanes
+// per row leave nothing to share (5-point 500^2 FP64 8.8 -> 9.5).
+uint32_t direct_split(uint32_t n_blk, uint32_t wave, bool wide_rows) {
+  uint32_t split = 1;
+  while (split < 16u && (uint64_t)n_blk * split * 2u <= wave) split *= 2;
+  const uint32_t last = n_blk % wave;  // blocks of the last wave
+  if (wide_rows && n_blk > wave && n_blk < 3u * wave && last && 5ull * last <= 3ull * wave) split = 2;
+  return split;
+}
+
 template <typename T>
 int csr_spmv(const mfp_csr_plan *plan, const T *data, const uint32_t *cols, const uint32_t *rp, const T *x,
              T *y, void *stream) {
@@ -777,10 +802,8 @@ int csr_spmv(const mfp_csr_plan *plan, const T *data, const uint32_t *cols, cons
     if (rest && !seq) { MFP_CSR_LAUNCH_N(2, false, rest) }
     if (vec) {
       auto k = seq ? d::csr_direct_kernel<T, true> : d::csr_direct_kernel<T, false>;
-      // few row blocks: several CTAs each, until the chip's 148 x 8 are in use
       const uint32_t n_blk = ceil_div(plan->rows, d::kBlock);
-      uint32_t split = 1;
-      while (split < 16u && n_blk * split * 2u <= 148u * 8u) split *= 2;
+      const uint32_t split = direct_split(n_blk, 148u * d::direct_ctas<T>(), plan->wide_rows[sizeof(T) == 8]);
       if (rest) {  // beside the blocks with longer rows
         const cudaError_t e = launch_after(k, n_blk * split, s, A, split);
         if (e != cudaSuccess) return cuda_fail(e, "csr_direct_kernel launch");

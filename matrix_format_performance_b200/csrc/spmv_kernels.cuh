@@ -1118,6 +1118,10 @@ __device__ __forceinline__ void csr_rows_direct(const csr_args<T> &A, uint64_t p
 #ifndef MFP_DIRECT_MINBLOCKS64
 #define MFP_DIRECT_MINBLOCKS64 6
 #endif
+template <typename T>
+constexpr uint32_t direct_ctas() {
+  return sizeof(T) == 4 ? MFP_DIRECT_MINBLOCKS : MFP_DIRECT_MINBLOCKS64;
+}
 // Row blocks in the plan's blk flags: bits 0 and 1 as in csr_args::blk, bits
 // 8-15 the lanes per row (FP32), bits 16-23 (FP64).  Blocks with a longer row and the long rows' pieces are
 // a csr_kernel launch of their own (their registers would weigh on this one),
@@ -1127,9 +1131,9 @@ __device__ __forceinline__ void csr_rows_direct(const csr_args<T> &A, uint64_t p
 // hold their place on an SM).
 // A row block is `split` CTAs that share its rounds (a power of two): on matrices
 // of few blocks the rounds one after the other are the time (20k rows of 4 to 64
-// elements, FP32: 16.2 us in 79 CTAs).
+// elements, FP32: 16.2 us in 79 CTAs), and on middle-sized ones the last wave.
 template <typename T, bool SEQ>
-__global__ void __launch_bounds__(kBlock, sizeof(T) == 4 ? MFP_DIRECT_MINBLOCKS : MFP_DIRECT_MINBLOCKS64)
+__global__ void __launch_bounds__(kBlock, direct_ctas<T>())
     csr_direct_kernel(const csr_args<T> A, uint32_t split) {
   const uint64_t pol = policy_evict_first();
   const uint32_t block = blockIdx.x / split, part = blockIdx.x % split;
