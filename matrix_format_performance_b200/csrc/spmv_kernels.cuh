@@ -909,8 +909,8 @@ __device__ __forceinline__ void csr_rowblock_main(const csr_args<T> &A, csr_smem
 // reduced from shared memory by power-of-two lane groups; a single-row bin is
 // reduced by the whole CTA straight from global memory; a single row above
 // the long threshold belongs to pieces.  SEQ (CSR scalar on short rows): the
-// same bins, each row summed by one thread in CSR order (rows above the
-// assist threshold by a warp).
+// same bins, each row summed by one thread in CSR order, also alone in a bin
+// (rows above the assist threshold by a warp, alone in a bin by the CTA).
 template <typename T, bool VEC, bool SEQ = false>
 __device__ __forceinline__ void csr_adaptive_main(const csr_args<T> &A, csr_smem<T> &sm, uint64_t pol,
                                                   uint32_t blk) {
@@ -919,7 +919,7 @@ __device__ __forceinline__ void csr_adaptive_main(const csr_args<T> &A, csr_smem
   const uint32_t t = threadIdx.x;
   if (nrows == 0) return;
   const uint32_t a = A.row_ptr[rb], b = A.row_ptr[re];
-  if (nrows == 1) {
+  if (nrows == 1 && (!SEQ || b - a > max(A.assist_thr, 8u))) {
     if (b - a > A.long_thr) return;
     acc_plain<T, VEC> acc;
     cta_range_dot<T, VEC>(A.vals, A.cols, A.x, a, b, acc, pol);

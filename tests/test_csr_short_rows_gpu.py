@@ -1,5 +1,5 @@
 """CSR row blocks read straight from global memory: every number of CTAs a block
-is split into."""
+is split into, and large matrices of which only part is such blocks."""
 import numpy as np
 import pytest
 
@@ -54,3 +54,17 @@ def test_every_split_of_a_row_block(oracle_lib, blocks, lo, hi, dtype):
     rng = np.random.default_rng(blocks)
     m = csr(rng.integers(lo, hi + 1, blocks * 256 - 17), 2_000, dtype)
     check(oracle_lib, m, synth.vector(1, m.cols).astype(dtype), 1)
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+def test_large_matrix_with_part_of_its_elements_in_short_row_blocks(oracle_lib, dtype):
+    """From 16M elements on, half of them in such blocks are enough; the other
+    blocks are a launch beside them."""
+    rng = np.random.default_rng(77)
+    lens = rng.integers(20, 50, 2000 * 256)
+    for b in rng.choice(2000, 600, replace=False):  # 30% of the blocks hold longer rows
+        lens[b * 256 + rng.integers(0, 256)] = rng.choice([65, 300, 3_000])
+    lens[1234 * 256] = 20_000
+    m = csr(lens, 50_000, dtype)
+    assert m.nnz >= 1 << 24
+    check(oracle_lib, m, synth.vector(2, m.cols).astype(dtype), 2)
