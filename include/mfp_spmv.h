@@ -217,7 +217,7 @@ int mfp_dev_csr_from_coo(int value_type, uint32_t rows, uint32_t cols, uint32_t 
 /* mfp_dev_csr_from_coo with a limit of its own on the sort's waits: a tile of
  * the radix sort looks at most `polls` times in vain for the counts of the tiles
  * before it (mfp_dev_csr_from_coo: 2^20, about a second).  A wait that runs out (0:
- * every one) ends the sort with MFP_ERROR_DEVICE_WAIT; the outputs then hold
+ * every one does) ends the sort with MFP_ERROR_DEVICE_WAIT; the outputs then hold
  * unspecified values and nothing is written beyond them. */
 int mfp_dev_csr_from_coo_limited(int value_type, uint32_t rows, uint32_t cols, uint32_t nnz, const uint32_t *row_ids,
                                  const uint32_t *col_ids, const double *values, uint32_t *row_ptr, uint32_t *columns,

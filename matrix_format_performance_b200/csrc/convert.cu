@@ -41,7 +41,7 @@ constexpr uint32_t kRadixBins = 1u << kRadixBits;
 static_assert(kRadixBins == kRadixThreads, "one thread per digit");
 constexpr uint32_t kRadixPasses = 8;                      // 64-bit keys
 constexpr uint32_t kRadixPolls = 1u << 20;                // look-back limit, about a second
-constexpr uint32_t kNoTile = 0xffffffffu;
+constexpr uint32_t kStop = 0x80000000u;                   // in a tile counter: no more tiles
 
 int cuda_fail(cudaError_t e, const char *what) {
   return fail(MFP_ERROR_CUDA, "%s: %s", what, cudaGetErrorString(e));
@@ -608,9 +608,9 @@ __device__ __forceinline__ uint32_t radix_excl(uint32_t v, uint32_t *s) {
   return (w ? s[w - 1] : 0u) + inc - v;
 }
 
-// Histograms of every digit: hist[pass][bin] (zeroed).  CHECK (triplets): err[0]
-// |= 1 (row id) / 2 (col id), err[1] = first bad element, err[2] = 1 when some
-// key is smaller than its predecessor (input not in CSR order).
+// Histograms of every digit: hist[pass][bin] (zeroed, as err).  CHECK (triplets):
+// err[0] |= 1 (row id) / 2 (col id), err[1] = ~ the first bad element, err[2] = 1
+// when some key is smaller than its predecessor (input not in CSR order).
 template <bool CHECK, uint32_t BITS, typename In>
 __global__ void __launch_bounds__(kThreads) radix_hist_kernel(uint32_t n, In in, uint32_t rows, uint32_t cols,
                                                               uint32_t passes, uint32_t *hist, uint32_t *err) {
@@ -644,7 +644,7 @@ __global__ void __launch_bounds__(kThreads) radix_hist_kernel(uint32_t n, In in,
         unsorted |= i < n && prev > k[j];
         if (bad[j]) {
           atomicOr(&err[0], in.r[i] >= rows ? 1u : 2u);
-          atomicMin(&err[1], (uint32_t)i);
+          atomicMax(&err[1], ~(uint32_t)i);
         }
       }
       if (i < n) {
@@ -670,13 +670,14 @@ __device__ __forceinline__ unsigned long long ld_status(const unsigned long long
   asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
   return v;
 }
-__device__ __forceinline__ uint32_t ld_word(const uint32_t *p) {
-  uint32_t v;
-  asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-  return v;
-}
 __device__ __forceinline__ void st_status(unsigned long long *p, unsigned long long v) {
   asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
+
+// A digit's look-back ran out: the error word, and no more tiles of later passes.
+__device__ __noinline__ void radix_give_up(uint32_t pass, uint32_t *counter, uint32_t *err) {
+  atomicOr(&err[3], 1u);
+  for (uint32_t p = pass + 1u; p < kRadixPasses; ++p) atomicOr(counter + (p - pass), kStop);
 }
 
 // One digit: stable scatter of a 6,144-key tile.  Keys go, in tile order, after
@@ -687,9 +688,11 @@ __device__ __forceinline__ void st_status(unsigned long long *p, unsigned long l
 // is placed in shared memory in digit order and written out as contiguous digit
 // runs; payloads follow through the same shared memory.  Tiles are numbered in
 // the order their CTAs start, so a tile only ever waits for CTAs that are
-// running.  The wait is bounded: a tile that gives up after `polls` looks sets
-// err[3] and scatters nothing (without its count its keys could land anywhere),
-// and what is launched or starts after that returns at once.
+// running.  The wait is bounded: a digit that gives up after `polls` looks in vain
+// goes on with the part of its count that it has, which is too small, so its keys
+// stay inside the array but leave holes in it; it sets err[3] and marks the tile
+// counters of the later passes (`counter` is this pass's of kRadixPasses), whose
+// tiles return at once instead of taking digits from the holes.
 struct radix_smem {
   unsigned long long key[kRadixTile];  // or payloads
   uint32_t wh[kRadixWarps][kRadixBins];
@@ -706,16 +709,14 @@ __global__ void __launch_bounds__(kRadixThreads, 2) radix_pass_kernel(uint32_t n
   radix_smem &S = *reinterpret_cast<radix_smem *>(smem_raw);
   constexpr uint32_t kPerWarp = kRadixTile / kRadixWarps;
   const uint32_t t = threadIdx.x, lane = t & 31u, warp = t >> 5;
-  if (t == 0) {
-    const uint32_t gave_up = ld_word(err + 3), at = atomicAdd(counter, 1u);
-    S.tile = gave_up ? kNoTile : at;
-  }
+  if (t == 0) S.tile = atomicAdd(counter, 1u);
 #pragma unroll
   for (uint32_t i = 0; i < kRadixWarps; ++i) S.wh[i][t] = 0u;
   const uint32_t hv = hist[t];
   __syncthreads();
-  const uint32_t tile = S.tile, shift = pass * BITS;
-  if (tile == kNoTile) return;
+  // (shuffled, so that the compiler knows the warp leaves as one: 18 us of 915)
+  const uint32_t tile = __shfl_sync(0xffffffffu, S.tile, 0), shift = pass * BITS;
+  if (tile & kStop) return;
   const uint64_t base = (uint64_t)tile * kRadixTile;
   const uint32_t tn = (uint32_t)min((uint64_t)kRadixTile, n - base);
   const uint32_t wbase = warp * kPerWarp + lane;
@@ -768,27 +769,26 @@ __global__ void __launch_bounds__(kRadixThreads, 2) radix_pass_kernel(uint32_t n
     }
   // the same digit's keys in earlier tiles
   uint32_t excl = 0;
-  bool found = tile == 0;
-  if (!found) {
+  if (tile) {
     const unsigned long long *st = status + t;
-    for (uint32_t w = tile - 1u; polls;) {
+    for (uint32_t w = tile - 1u, waits = 0;;) {
       const unsigned long long v = ld_status(st + (size_t)w * kRadixBins);
       const uint32_t flag = (uint32_t)(v >> 32);
-      if (flag <= 2u * pass) {  // not there yet
-        --polls;
+      if (flag <= 2u * pass || polls == 0u) {  // not there yet
+        if (++waits > polls) {
+          radix_give_up(pass, counter, err);
+          break;
+        }
         continue;
       }
       excl += (uint32_t)v;
-      if ((found = flag == 2u * pass + 2u || w == 0)) break;
+      if (flag == 2u * pass + 2u || w == 0) break;
       --w;
     }
-    if (found) st_status(mine, status_word(pass, true, excl + tot));
+    st_status(mine, status_word(pass, true, excl + tot));
   }
   S.gbase[t] = below + excl - start;
-  if (__syncthreads_or(!found)) {
-    if (t == 0) atomicOr(&err[3], 1u);
-    return;
-  }
+  __syncthreads();
   uint32_t g[kRadixRounds];
 #pragma unroll
   for (uint32_t j = 0; j < kRadixRounds; ++j) {
@@ -821,8 +821,9 @@ __global__ void __launch_bounds__(kThreads) rowptr_from_rows_kernel(uint32_t nnz
                                                                     const uint32_t *__restrict__ ri, uint32_t *rp,
                                                                     const uint32_t *err) {
   const uint64_t p = (uint64_t)blockIdx.x * kThreads + threadIdx.x;
-  if (p > nnz || __ldg(err + 3)) return;
+  if (p > nnz) return;
   const row_span span = rows_starting_at(p, nnz, p ? ri[p - 1] : 0u, p < nnz ? ri[p] : 0u, rows);
+  if (__ldg(err + 3)) return;
   for (uint64_t q = span.first; q < span.end; ++q) rp[q] = (uint32_t)p;
 }
 
@@ -873,34 +874,47 @@ int coo_from_csr_t(uint32_t rows, const uint32_t *rp, const uint32_t *ci, const 
   return ok();
 }
 
-// Device words of one sort: histograms, tile counters and status words, zeroed
-// by begin().
+// Device words of one sort, zeroed by begin(): status words, histograms, tile
+// counters and error words, each from a 128-byte boundary (whole warps read a
+// tile's row of status words: 48 bytes off, a pass took 4% longer).
 struct radix_state {
-  uint32_t *hist = nullptr, *counters = nullptr;
   unsigned long long *status = nullptr;
+  uint32_t *err = nullptr, *hist = nullptr, *counters = nullptr;
   uint32_t tiles = 0;
-  int begin(uint32_t n, const radix_digits &dg, scratch &sc) {
+  int begin(uint32_t n, scratch &sc) {
     tiles = blocks_for(n, kRadixTile);
-    const size_t words = (size_t)tiles * kRadixBins;
-    const size_t bytes = words * 8u + kRadixPasses * (kRadixBins + 1u) * 4u;
+    const size_t words = (size_t)tiles * kRadixBins, bytes = words * 8u + (kRadixPasses * kRadixBins + 32u + 4u) * 4u;
     unsigned char *p = nullptr;
     const int s = sc.get(&p, bytes);
     if (s) return s;
     status = reinterpret_cast<unsigned long long *>(p);
     hist = reinterpret_cast<uint32_t *>(p + words * 8u);
     counters = hist + kRadixPasses * kRadixBins;
+    err = counters + 32;
     CV_TRY(cudaMemsetAsync(p, 0, bytes, sc.st), "cudaMemsetAsync");
     return MFP_SUCCESS;
   }
 };
+// The histograms of `in`, with the other device words made ready.
+template <bool CHECK, typename In>
+int radix_histograms(uint32_t n, const In &in, uint32_t rows, uint32_t cols, const radix_digits &dg, radix_state &R,
+                     scratch &sc) {
+  const int s = R.begin(n, sc);
+  if (s) return s;
+  auto k = dg.bits == 8u ? radix_hist_kernel<CHECK, 8, In> : radix_hist_kernel<CHECK, 9, In>;
+  k<<<std::min(kKeyBlocks, blocks_for(n, 4u * kThreads)), kThreads, 0, sc.st>>>(
+      n, in, rows, cols, dg.passes, R.hist, R.err);
+  CV_TRY(cudaGetLastError(), "radix_hist_kernel");
+  return MFP_SUCCESS;
+}
 template <typename P, typename In, typename Out>
 int radix_pass(uint32_t n, const In &in, const Out &out, const radix_digits &dg, uint32_t pass, const radix_state &R,
-               uint32_t polls, uint32_t *err, scratch &sc) {
+               uint32_t polls, scratch &sc) {
   auto k = dg.bits == 8u ? radix_pass_kernel<8, P, In, Out> : radix_pass_kernel<9, P, In, Out>;
   CV_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(radix_smem)),
          "cudaFuncSetAttribute");
   k<<<R.tiles, kRadixThreads, sizeof(radix_smem), sc.st>>>(n, in, out, pass, R.hist + pass * kRadixBins,
-                                                           R.counters + pass, R.status, polls, err);
+                                                           R.counters + pass, R.status, polls, R.err);
   CV_TRY(cudaGetLastError(), "radix_pass_kernel");
   return MFP_SUCCESS;
 }
@@ -916,21 +930,18 @@ int radix_sort_pairs(uint32_t n, uint32_t bits, unsigned long long *&k0, P *&p0,
   const radix_digits dg(bits);
   unsigned long long *k1 = nullptr;
   P *p1 = nullptr;
-  uint32_t *err = nullptr, h_err[4];
+  uint32_t h_err[4];
   radix_state R;
   int s;
-  if ((s = sc.get(&k1, n)) || (s = sc.get(&p1, n)) || (s = sc.get(&err, 4)) || (s = R.begin(n, dg, sc))) return s;
-  CV_TRY(cudaMemsetAsync(err, 0, 16, sc.st), "cudaMemsetAsync");
-  auto hk = dg.bits == 8u ? radix_hist_kernel<false, 8, pairs_in<P>> : radix_hist_kernel<false, 9, pairs_in<P>>;
-  hk<<<std::min(kKeyBlocks, blocks_for(n, 4u * kThreads)), kThreads, 0, sc.st>>>(n, pairs_in<P>{k0, p0}, 0u, 0u,
-                                                                                 dg.passes, R.hist, err);
-  CV_TRY(cudaGetLastError(), "radix_hist_kernel");
+  if ((s = sc.get(&k1, n)) || (s = sc.get(&p1, n)) ||
+      (s = radix_histograms<false>(n, pairs_in<P>{k0, p0}, 0u, 0u, dg, R, sc)))
+    return s;
   for (uint32_t pass = 0; pass < dg.passes; ++pass) {
-    if ((s = radix_pass<P>(n, pairs_in<P>{k0, p0}, pairs_out<P>{k1, p1}, dg, pass, R, kRadixPolls, err, sc))) return s;
+    if ((s = radix_pass<P>(n, pairs_in<P>{k0, p0}, pairs_out<P>{k1, p1}, dg, pass, R, kRadixPolls, sc))) return s;
     std::swap(k0, k1);
     std::swap(p0, p1);
   }
-  CV_TRY(cudaMemcpyAsync(h_err, err, sizeof(h_err), cudaMemcpyDeviceToHost, sc.st), "cudaMemcpyAsync");
+  CV_TRY(cudaMemcpyAsync(h_err, R.err, sizeof(h_err), cudaMemcpyDeviceToHost, sc.st), "cudaMemcpyAsync");
   CV_TRY(cudaStreamSynchronize(sc.st), "cudaStreamSynchronize");
   return radix_error(h_err[3]);
 }
@@ -970,21 +981,14 @@ int csr_from_coo_t(uint32_t rows, uint32_t cols, uint32_t nnz, const uint32_t *r
   }
   const uint32_t rb = rows > 1 ? bits_for(rows - 1) : 0u, cb = cols > 1 ? bits_for(cols - 1) : 0u;
   const radix_digits dg(rb + cb);
-  uint32_t *err = nullptr;
   radix_state R;
   int s;
-  if ((s = sc.get(&err, 4)) || (s = R.begin(nnz, dg, sc))) return s;
-  const uint32_t err_init[4] = {0u, 0xffffffffu, 0u, 0u};
-  CV_TRY(cudaMemcpyAsync(err, err_init, sizeof(err_init), cudaMemcpyHostToDevice, st), "cudaMemcpyAsync");
-  auto hk = dg.bits == 8u ? radix_hist_kernel<true, 8, triplets_in<T>> : radix_hist_kernel<true, 9, triplets_in<T>>;
-  hk<<<std::min(kKeyBlocks, blocks_for(nnz, 4u * kThreads)), kThreads, 0, st>>>(nnz, triplets_in<T>{ri, ci, v, cb}, rows,
-                                                                                cols, dg.passes, R.hist, err);
-  CV_TRY(cudaGetLastError(), "radix_hist_kernel");
+  if ((s = radix_histograms<true>(nnz, triplets_in<T>{ri, ci, v, cb}, rows, cols, dg, R, sc))) return s;
   uint32_t h_err[4];
-  CV_TRY(cudaMemcpyAsync(h_err, err, sizeof(h_err), cudaMemcpyDeviceToHost, st), "cudaMemcpyAsync");
+  CV_TRY(cudaMemcpyAsync(h_err, R.err, sizeof(h_err), cudaMemcpyDeviceToHost, st), "cudaMemcpyAsync");
   CV_TRY(cudaStreamSynchronize(st), "cudaStreamSynchronize");
-  if (h_err[0] & 1u) return fail(MFP_ERROR_INVALID_VALUE, "row id >= rows %u at element %u", rows, h_err[1]);
-  if (h_err[0] & 2u) return fail(MFP_ERROR_INVALID_VALUE, "col id >= cols %u at element %u", cols, h_err[1]);
+  if (h_err[0] & 1u) return fail(MFP_ERROR_INVALID_VALUE, "row id >= rows %u at element %u", rows, ~h_err[1]);
+  if (h_err[0] & 2u) return fail(MFP_ERROR_INVALID_VALUE, "col id >= cols %u at element %u", cols, ~h_err[1]);
   // a kernel that reads the triplets and writes the CSR needs them apart (several
   // passes read them all into scratch first)
   if (!h_err[2] || dg.passes == 1u) {
@@ -1010,18 +1014,19 @@ int csr_from_coo_t(uint32_t rows, uint32_t cols, uint32_t nnz, const uint32_t *r
       const pairs_in<T> mid_in{k[(pass + 1u) & 1u], p[(pass + 1u) & 1u]};
       const pairs_out<T> mid_out{k[pass & 1u], p[pass & 1u]};
       if (first)
-        s = last ? radix_pass<T>(nnz, in, out, dg, pass, R, polls, err, sc)
-                 : radix_pass<T>(nnz, in, mid_out, dg, pass, R, polls, err, sc);
+        s = last ? radix_pass<T>(nnz, in, out, dg, pass, R, polls, sc)
+                 : radix_pass<T>(nnz, in, mid_out, dg, pass, R, polls, sc);
       else
-        s = last ? radix_pass<T>(nnz, mid_in, out, dg, pass, R, polls, err, sc)
-                 : radix_pass<T>(nnz, mid_in, mid_out, dg, pass, R, polls, err, sc);
+        s = last ? radix_pass<T>(nnz, mid_in, out, dg, pass, R, polls, sc)
+                 : radix_pass<T>(nnz, mid_in, mid_out, dg, pass, R, polls, sc);
       if (s) return s;
     }
     sorted_rows = out_rows;
   }
-  rowptr_from_rows_kernel<<<blocks_for((uint64_t)nnz + 1, kThreads), kThreads, 0, st>>>(nnz, rows, sorted_rows, rp, err);
+  rowptr_from_rows_kernel<<<blocks_for((uint64_t)nnz + 1, kThreads), kThreads, 0, st>>>(nnz, rows, sorted_rows, rp, R.err);
   CV_TRY(cudaGetLastError(), "rowptr_from_rows_kernel");
-  CV_TRY(cudaMemcpyAsync(h_err, err, sizeof(h_err), cudaMemcpyDeviceToHost, st), "cudaMemcpyAsync");
+  if (h_err[2])  // sorted here: whether a tile gave up
+    CV_TRY(cudaMemcpyAsync(h_err, R.err, sizeof(h_err), cudaMemcpyDeviceToHost, st), "cudaMemcpyAsync");
   CV_TRY(cudaStreamSynchronize(st), "cudaStreamSynchronize");
   if (h_err[3]) return radix_error(h_err[3]);
   return ok();
