@@ -620,8 +620,9 @@ int mfp_matrix_spmv(const mfp_matrix *m, const void *x, void *y, void *stream);
  * waits for the copy.  Page-locked host buffers give full PCIe bandwidth.
  * When host_y is page-locked and device-addressable and the format's kernel
  * stores each row of y once in row order (CSR scalar / adaptive, CSR vector
- * with lanes per row, ELL, SCOO, the reduced-precision layouts), the kernel
- * stores y straight into host_y, so the copy-out overlaps the kernel.
+ * with lanes per row, ELL, SCOO unless a slice takes longer than kernel and copy
+ * one after the other, the reduced-precision layouts), the kernel stores y
+ * straight into host_y, so the copy-out overlaps the kernel.
  * The host-buffer calls stage through buffers owned by the handle: one such
  * call at a time per handle. */
 int mfp_matrix_spmv_host(mfp_matrix *m, const void *host_x, void *host_y, void *stream);

@@ -1424,6 +1424,7 @@ struct mfp_matrix {
   d::scoo_tile *tiles = nullptr;      // row-ordered SCOO: the slices' warp tiles
   call_blocks carry_ws;               // their carries, per call
   uint32_t n_tiles = 0;
+  bool host_slices = false;           // one CTA per slice for y in page-locked host memory (scoo_host_slices)
   bool long_rows = false;             // reduced-precision CSR: a row longer than kLowpTmaMaxRow
 };
 
@@ -1608,10 +1609,28 @@ bool scoo_use_tiles(const mfp_matrix *m, const uint32_t *sp_host) {
   return (used < 148u * 4u || mean < 16 * d::kWarpTile) && m->nnz >= 148u * 6u * d::kWarpTile * 4u;
 }
 
+// Whether a tiled handle's y goes to page-locked host memory by one CTA per slice,
+// which stores it there as the slices finish, rather than by the tiles and a copy
+// after them: when the slowest of the heaviest slice, the product and the copy
+// takes less than product and copy one after the other.  B200, PCIe at 55 GB/s,
+// power-law 4M rows with host vectors: FP32 720 us against 791, FP64 1,331 against
+// 1,420; 5-point 700^2 FP64 181 against 196; but 50k rows FP32, whose heaviest
+// slice takes 49 us, 77 against 46.  The rates: 256 elements of a slice's CTA
+// 0.25 us in FP32 and 0.5 in FP64, all CTAs together 5.4 and 7.5 us per million
+// elements.
+bool scoo_host_slices(const mfp_matrix *m, uint64_t heaviest) {
+  const bool f64 = m->value_type == MFP_F64;
+  const double slice = heaviest * (f64 ? 0.5 : 0.25) / d::kWarpTile, product = m->nnz * (f64 ? 7.5e-6 : 5.4e-6);
+  const double copy = (double)m->rows * (f64 ? 8 : 4) / 55e3;
+  return std::max(slice, product) < product + copy;
+}
+
 // Row-ordered SCOO: every slice's 256-element tiles (an entry without elements
-// for an empty slice, whose rows it zeroes) and the scratch of their carries.
+// for an empty slice, whose rows it zeroes) and the scratch of their carries, and
+// the slices by element count for calls that run one CTA per slice.
 int scoo_attach_tiles(mfp_matrix *m, const uint32_t *sp_host) {
   std::vector<d::scoo_tile> t;
+  uint64_t heaviest = 0;
   t.reserve((size_t)m->nnz / d::kWarpTile + m->slices);
   for (uint32_t s = 0; s < m->slices && (uint64_t)s * m->slice_size < m->rows; ++s) {
     const uint32_t eb = sp_host[s], ee = sp_host[s + 1];
@@ -1619,6 +1638,7 @@ int scoo_attach_tiles(mfp_matrix *m, const uint32_t *sp_host) {
       t.push_back({0u, 0u, s, d::kSliceEmpty});
       continue;
     }
+    heaviest = std::max<uint64_t>(heaviest, ee - eb);
     for (uint32_t g0 = eb & ~7u; g0 < ee;) {
       const uint32_t c1 = ee - g0 > d::kWarpTile ? g0 + d::kWarpTile : ee;
       const bool first = g0 <= eb;
@@ -1627,11 +1647,19 @@ int scoo_attach_tiles(mfp_matrix *m, const uint32_t *sp_host) {
     }
   }
   m->n_tiles = (uint32_t)t.size();
+  m->host_slices = scoo_host_slices(m, heaviest);
+  // one allocation: the tiles, then the order
+  t.resize(t.size() + ((size_t)m->slices + 3u) / 4u);
+  uint32_t *order = reinterpret_cast<uint32_t *>(t.data() + m->n_tiles);
+  int st = mfp_scoo_slice_order(m->slices, sp_host, order);
+  if (st) return st;
   const cudaError_t e = m->carry_ws.init(carry_ws_bytes(m->n_tiles), 0, &m->device_bytes);
   if (e != cudaSuccess)
     return fail(e == cudaErrorMemoryAllocation ? MFP_ERROR_OUT_OF_MEMORY : MFP_ERROR_CUDA, "SCOO carries: %s",
                 cudaGetErrorString(e));
-  return track_upload(m, &m->tiles, t.data(), t.size());
+  if ((st = track_upload(m, &m->tiles, t.data(), t.size()))) return st;
+  m->order = reinterpret_cast<uint32_t *>(m->tiles + m->n_tiles);
+  return MFP_SUCCESS;
 }
 
 int check_columns(const uint32_t *c, uint64_t n, uint32_t cols) {
@@ -2102,7 +2130,8 @@ int mfp_matrix_get_info(const mfp_matrix *m, mfp_matrix_info *out) {
   return ok();
 }
 
-int mfp_matrix_spmv(const mfp_matrix *m, const void *x, void *y, void *stream) {
+// to_host: y is page-locked host memory
+static int matrix_spmv(const mfp_matrix *m, const void *x, void *y, void *stream, bool to_host) {
   if (!m || !y || (!x && m->cols)) return fail(MFP_ERROR_INVALID_VALUE, "null argument");
   const bool f64 = m->value_type == MFP_F64;
   switch (m->format) {
@@ -2133,7 +2162,7 @@ int mfp_matrix_spmv(const mfp_matrix *m, const void *x, void *y, void *stream) {
                    : scoo_spmv<float, true>(m->rows, m->slices, m->slice_size, (const float *)m->vals, m->cols_a,
                                             m->rows_a, m->aux, m->win, m->max_window, m->order, (const float *)x,
                                             (float *)y, stream);
-      if (m->tiles) {
+      if (m->tiles && !to_host) {
         const call_scratch ws(m->carry_ws, as_stream(stream));
         if (ws.ptr())  // without memory for the carries: one CTA per slice
           return f64 ? scoo_tile_spmv<double>(m->rows, m->slice_size, m->n_tiles, m->tiles, (const double *)m->vals,
@@ -2167,6 +2196,10 @@ int mfp_matrix_spmv(const mfp_matrix *m, const void *x, void *y, void *stream) {
   }
 }
 
+int mfp_matrix_spmv(const mfp_matrix *m, const void *x, void *y, void *stream) {
+  return matrix_spmv(m, x, y, stream, false);
+}
+
 // Formats whose kernels write each row of y once, a warp's stores covering
 // consecutive rows: their y can go straight into a page-locked host buffer.
 static bool writes_y_in_row_order(const mfp_matrix *m) {
@@ -2178,7 +2211,7 @@ static bool writes_y_in_row_order(const mfp_matrix *m) {
     case MFP_FORMAT_SCOO:
     case MFP_FORMAT_CSR_LOWP:
     case MFP_FORMAT_ELL_LOWP:
-      return !(m->plan && m->plan->tile) && !m->rows_unsorted && !m->tiles;
+      return !(m->plan && m->plan->tile) && !m->rows_unsorted && (!m->tiles || m->host_slices);
     case MFP_FORMAT_CSR_VECTOR:
       return !(m->plan && m->plan->tile);
     default:  // COO and the warp-tile kernels write rows as their tiles finish; the hybrid adds into y
@@ -2203,7 +2236,7 @@ int mfp_matrix_spmv_host(mfp_matrix *m, const void *hx, void *hy, void *stream) 
   }
   if (m->cols)
     CUDA_TRY(cudaMemcpyAsync(m->dx, hx, (size_t)m->cols * vs, cudaMemcpyHostToDevice, s), "cudaMemcpyAsync x");
-  int st = mfp_matrix_spmv(m, m->dx, y_mapped ? y_mapped : m->dy, stream);
+  int st = matrix_spmv(m, m->dx, y_mapped ? y_mapped : m->dy, stream, y_mapped != nullptr);
   if (st) return st;
   if (m->rows && !y_mapped)
     CUDA_TRY(cudaMemcpyAsync(hy, m->dy, (size_t)m->rows * vs, cudaMemcpyDeviceToHost, s), "cudaMemcpyAsync y");

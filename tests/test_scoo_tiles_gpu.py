@@ -75,3 +75,31 @@ def test_slices_beyond_shared_memory_are_refused(dtype):
     with pytest.raises(MfpError, match="too large for shared memory"):
         handle_spmv(dm, m, np.ones(100, dtype))
     dm.close()
+
+
+def pinned(n, dtype):
+    return torch.full((n,), float("nan"), dtype=torch.float32 if dtype == np.float32 else torch.float64).pin_memory()
+
+
+@pytest.mark.parametrize("longest", [64, 20_000])  # many rows and even slices; few rows and a heavy slice
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+def test_host_vectors(oracle_lib, longest, dtype):
+    """A tiled handle's product with host vectors, y page-locked or not, has the
+    bits of the device call, whichever kernel stores it."""
+    rng = np.random.default_rng(longest)
+    rows = 400_000 if longest == 64 else 3_000
+    lens = rng.integers(0, 6, rows)
+    lens[rows // 2] = longest
+    rp = np.concatenate([[0], np.cumsum(lens)]).astype(np.uint32)
+    m = F.csr_matrix_class.from_arrays(rows, rows, rp, rng.integers(0, rows, int(rp[-1])).astype(np.uint32),
+                                       rng.uniform(-1, 1, int(rp[-1])), dtype)
+    dm = DeviceMatrix.build(m, SCOO)
+    assert dm.info().kernel_launches == 2  # tiles and fix-up
+    x = rng.uniform(-1, 1, rows).astype(dtype)
+    want = handle_spmv(dm, m, x)
+    ys, ab = oracle_lib.csr_spmv_exact(m.rows, m.row_ptr, m.columns, m.data, x)
+    assert np.all(np.abs(want.astype(np.float64) - ys) <= {np.float32: 1e-5, np.float64: 1e-12}[dtype] * ab)
+    for y in (pinned(rows, dtype).numpy(), np.full(rows, np.nan, dtype)):
+        dm.spmv_host(x, y)
+        assert np.array_equal(y.view(np.uint8), want.view(np.uint8))
+    dm.close()
