@@ -29,7 +29,7 @@ ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 CU_SOURCES = ["capi.cu", "convert.cu"]
 CPP_SOURCES = ["util.cpp", "scratch.cpp", "formats.cpp", "synth.cpp"]
 HEADERS = ["spmv_device.cuh", "spmv_kernels.cuh", "spmv_stream.cuh", "spmv_lowp.cuh", "mlp.cuh", "host_common.h",
-           "scratch.h", "row_span.h"]
+           "scratch.h", "row_span.h", "quads.h"]
 
 NVCC_FLAGS = ARCH + ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-Xptxas", "-O3",
                      "--expt-relaxed-constexpr", f"-I{ROOT / 'include'}"]

@@ -32,6 +32,7 @@
 // run as extra CTAs of the same launch and meet in a partial-sum buffer.
 #pragma once
 
+#include "quads.h"
 #include "spmv_device.cuh"
 
 namespace mfp {
@@ -1037,7 +1038,7 @@ template <typename T>
 __device__ __forceinline__ void load_quad(const csr_args<T> &A, uint32_t e, uint32_t re, row_quad<T> &q, uint64_t pol) {
   q.e = e;
   if (e >= re) return;
-  if (e + 4u <= A.nnz) {
+  if (whole_quad(e, A.nnz)) {
     ld_stream4(A.vals + e, q.v, pol);
     ld_stream4(A.cols + e, q.c, pol);
   } else {
