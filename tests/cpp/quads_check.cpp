@@ -1,5 +1,6 @@
 // quads.h for every remainder of the last quad, up to 2^32 - 1 elements.
 #include <cstdio>
+#include <initializer_list>
 
 #include "../../matrix_format_performance_b200/csrc/quads.h"
 
