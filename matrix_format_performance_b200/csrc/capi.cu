@@ -240,7 +240,7 @@ bool auto_config(const mfp_csr_config *c) {
   return !c || memcmp(c, &none, sizeof(none)) == 0;
 }
 constexpr uint32_t kDefaultLong = 4096;
-constexpr uint32_t kDirectMixed = 16u << 20;
+constexpr uint32_t kDirectMixed = 64u << 20;
 constexpr uint32_t kDefaultAssist = 64;
 
 // Row blocks of 256 rows: element range and, in z, bit 0 a long row, bit 1 an
@@ -264,7 +264,7 @@ bool row_blocks_regular(uint32_t rows, const uint32_t *rp) {
     seen += rp[r1] - rp[r0];
     regular += all_short ? rp[r1] - rp[r0] : 0u;
   }
-  return 5 * regular >= 2 * seen;  // 40%: the plan asks for half of all
+  return 5 * regular >= 2 * seen;  // 40%: the plan asks for at least half of all
 }
 std::vector<uint4> row_block_info(uint32_t rows, const uint32_t *rp, uint32_t long_thr, uint32_t assist_thr,
                                   uint64_t *regular) {
@@ -409,8 +409,9 @@ int build_stream_plans(mfp_csr_plan *plan, const uint32_t *rp) {
   return MFP_SUCCESS;
 }
 
-extern "C" int mfp_csr_plan_create(uint32_t rows, uint32_t cols, uint32_t nnz, const uint32_t *rp,
-                                   int algo, const mfp_csr_config *config, mfp_csr_plan **out) {
+// value_type: MFP_F32 / MFP_F64 where the caller knows it, else -1.
+static int csr_plan_create(int value_type, uint32_t rows, uint32_t cols, uint32_t nnz, const uint32_t *rp, int algo,
+                           const mfp_csr_config *config, mfp_csr_plan **out) {
   if (!out) return fail(MFP_ERROR_INVALID_VALUE, "plan output is NULL");
   *out = nullptr;
   if (algo < 0 || algo > 2) return fail(MFP_ERROR_INVALID_VALUE, "unknown CSR algorithm %d", algo);
@@ -434,11 +435,12 @@ extern "C" int mfp_csr_plan_create(uint32_t rows, uint32_t cols, uint32_t nnz, c
   // 27-point stencil, banded 8M) a bin holds too few rows for its threads.
   const bool exact = cfg.long_row_threshold == UINT32_MAX && cfg.assist_threshold == UINT32_MAX;
   plan->binned = algo == MFP_CSR_SCALAR && cfg.kernel == 0 && !exact && rows && (double)nnz / rows < 16.0;
-  // Automatic plans with nearly all elements, or half of many, in row blocks
-  // without a row above 64 elements: those rows straight from global memory, the
-  // others in the CSR-Adaptive bins beside them (two launches: 64 uneven matrices
-  // of 72M nonzeros 249 -> 230 us, 40 of 36M 123 -> 113, but 14 of 8M 32.4 -> 34.7
-  // and 20 of 15M in FP64 74 -> 82).  B200 against the row blocks / bins / warp
+  // Automatic plans with nearly all elements, or in FP32 half of many, in row
+  // blocks without a row above 64 elements: those rows straight from global memory,
+  // the others in the CSR-Adaptive bins beside them (two launches).  Batches of 40
+  // to 64 uneven matrices, bins alone -> both, FP32: from 64M elements 228 -> 218 us
+  // (78M), 232 -> 223 (71M), 208 -> 208 (69M), but between 92 -> 97 (35M), 128 -> 137
+  // (49M) and 178 -> 169 (53M) below; FP64 172 -> 181 (47M), 353 -> 363 (83M).  B200 against the row blocks / bins / warp
   // tiles, inputs changing from pass to pass: banded 8M rows FP32 scalar 400 ->
   // 361 us, vector 539 -> 341, 4M rows FP64 scalar 351 -> 275; 27-point 128^3 FP32
   // scalar 121 -> 107, Adaptive 135 -> 97, 101^3 FP64 vector 96 -> 73; 5-point
@@ -449,7 +451,7 @@ extern "C" int mfp_csr_plan_create(uint32_t rows, uint32_t cols, uint32_t nnz, c
   if (MFP_CSR_DIRECT && automatic && nnz && row_blocks_regular(rows, rp)) {
     uint64_t regular = 0;
     blk = row_block_info(rows, rp, kDefaultLong, kDefaultAssist, &regular);
-    plan->direct = 16 * regular >= 15ull * nnz || (2 * regular >= nnz && nnz >= kDirectMixed);
+    plan->direct = 16 * regular >= 15ull * nnz || (value_type == MFP_F32 && nnz >= kDirectMixed && 2 * regular >= nnz);
     if (plan->direct) {
       plan->binned = false;
       uint64_t wide[2] = {0, 0};
@@ -632,6 +634,11 @@ extern "C" int mfp_csr_plan_create(uint32_t rows, uint32_t cols, uint32_t nnz, c
   }
   *out = plan;
   return ok();
+}
+
+extern "C" int mfp_csr_plan_create(uint32_t rows, uint32_t cols, uint32_t nnz, const uint32_t *rp, int algo,
+                                   const mfp_csr_config *config, mfp_csr_plan **out) {
+  return csr_plan_create(-1, rows, cols, nnz, rp, algo, config, out);
 }
 
 extern "C" int mfp_csr_plan_destroy(mfp_csr_plan *plan) {
@@ -1707,7 +1714,7 @@ int mfp_matrix_create_csr(int format, int vt, uint32_t rows, uint32_t cols, uint
   m->format_bytes = (uint64_t)nnz * (vs + 4) + ((uint64_t)rows + 1) * 4 + (uint64_t)cols * vs + (uint64_t)rows * vs;
   if ((st = track_upload_bytes(m, &m->vals, data, (size_t)nnz * vs)) ||
       (st = track_upload(m, &m->cols_a, ci, nnz)) || (st = track_upload(m, &m->rows_a, rp, (size_t)rows + 1)) ||
-      (st = mfp_csr_plan_create(rows, cols, nnz, rp, format, cfg, &m->plan))) {
+      (st = csr_plan_create(vt, rows, cols, nnz, rp, format, cfg, &m->plan))) {
     mfp_matrix_destroy(m);
     return st;
   }
@@ -1929,7 +1936,7 @@ int mfp_matrix_create_device(int format, int vt, uint32_t rows, uint32_t cols, u
           cudaMemcpy(m->rows_a, rp, hrp.size() * 4, cudaMemcpyDeviceToDevice) != cudaSuccess ||
           cudaMemcpy(hrp.data(), rp, hrp.size() * 4, cudaMemcpyDeviceToHost) != cudaSuccess)
         return bail(fail(MFP_ERROR_CUDA, "cudaMemcpy CSR arrays"));
-      if ((st = mfp_csr_plan_create(rows, cols, nnz, hrp.data(), format, o.csr, &m->plan))) return bail(st);
+      if ((st = csr_plan_create(vt, rows, cols, nnz, hrp.data(), format, o.csr, &m->plan))) return bail(st);
       m->device_bytes += m->plan->device_bytes;
       break;
     }
@@ -2441,7 +2448,7 @@ void batch_drop_graph(mfp_batch *b) {
 }
 int batch_plan(mfp_batch *b, const mfp_batch_config &c, mfp_csr_plan **out) {
   if (c.algo < 0 || c.algo > 2) return fail(MFP_ERROR_INVALID_VALUE, "batch algo must be 0, 1 or 2");
-  return mfp_csr_plan_create(b->rows, b->cols, b->nnz, b->host_rp.data(), c.algo, &c.csr, out);
+  return csr_plan_create(b->vt, b->rows, b->cols, b->nnz, b->host_rp.data(), c.algo, &c.csr, out);
 }
 int batch_launch(const mfp_batch *b, const mfp_csr_plan *plan, const void *x, void *y, void *stream) {
   return b->vt == MFP_F64 ? csr_spmv<double>(plan, (const double *)b->vals, b->cols_a, b->rp, (const double *)x,

@@ -56,15 +56,39 @@ def test_every_split_of_a_row_block(oracle_lib, blocks, lo, hi, dtype):
     check(oracle_lib, m, synth.vector(1, m.cols).astype(dtype), 1)
 
 
-@pytest.mark.parametrize("dtype", [np.float32, np.float64])
-def test_large_matrix_with_part_of_its_elements_in_short_row_blocks(oracle_lib, dtype):
-    """From 16M elements on, half of them in such blocks are enough; the other
-    blocks are a launch beside them."""
-    rng = np.random.default_rng(77)
-    lens = rng.integers(20, 50, 2000 * 256)
-    for b in rng.choice(2000, 600, replace=False):  # 30% of the blocks hold longer rows
+def part_short(blocks, rng):
+    """Rows of 20 to 49 elements; 30% of the row blocks hold a longer one too."""
+    lens = rng.integers(20, 50, blocks * 256)
+    for b in rng.choice(blocks, blocks * 3 // 10, replace=False):
         lens[b * 256 + rng.integers(0, 256)] = rng.choice([65, 300, 3_000])
     lens[1234 * 256] = 20_000
+    return lens
+
+
+def test_large_matrix_with_part_of_its_elements_in_short_row_blocks(oracle_lib):
+    """FP32 from 64M elements on: half of them in such blocks are enough, the other
+    blocks are a launch beside them."""
+    m = csr(part_short(7_600, np.random.default_rng(77)), 50_000, np.float32)
+    assert m.nnz >= 64 << 20
+    check(oracle_lib, m, synth.vector(2, m.cols).astype(np.float32), 2)
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+def test_middle_sized_matrix_with_part_of_its_elements_in_short_row_blocks(oracle_lib, dtype):
+    """Below that, and in FP64: one kernel for all blocks (vector: two passes)."""
+    m = csr(part_short(2_000, np.random.default_rng(78)), 50_000, dtype)
+    x = synth.vector(2, m.cols).astype(dtype)
+    check(oracle_lib, m, x, None)
+    for fmt, launches in ((CSR_SCALAR, 1), (CSR_VECTOR, 2), (CSR_ADAPTIVE, 1)):
+        spmv(m, fmt, x, launches)
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+def test_short_rows_alone_in_a_bin(oracle_lib, dtype):
+    """Rows of up to 64 elements between two that fill a bin each."""
+    rng = np.random.default_rng(79)
+    lens = rng.integers(20, 50, 1000 * 256)
+    for b in range(0, 1000, 50):
+        lens[b * 256:b * 256 + 7] = [rng.integers(30, 65), 2_500, 64, 4_000, 1, 2_300, 40]
     m = csr(lens, 50_000, dtype)
-    assert m.nnz >= 1 << 24
     check(oracle_lib, m, synth.vector(2, m.cols).astype(dtype), 2)
