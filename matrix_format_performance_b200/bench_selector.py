@@ -114,8 +114,8 @@ def main() -> None:
     ap.add_argument("--big-cap", type=int, default=1 << 26)
     ap.add_argument("--out", default="selector_out")
     ap.add_argument("--dataset", default=None)
-    ap.add_argument("--epochs", type=int, default=400)
-    ap.add_argument("--members", type=int, default=10)
+    ap.add_argument("--epochs", type=int, default=800)
+    ap.add_argument("--members", type=int, default=20)
     a = ap.parse_args()
     import torch
 
