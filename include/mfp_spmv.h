@@ -567,7 +567,8 @@ int mfp_matrix_create_coo(int value_type, uint32_t rows, uint32_t cols, uint32_t
  * in any order (the sort_cols layout, detected here: SpMV then uses the
  * shared-memory-atomics kernel).  Row-ordered slices that are uneven, few or
  * short run as independent 256-element warp tiles and a fix-up launch instead
- * of one CTA per slice: the same tiles and the same bits. */
+ * of one CTA per slice: the same tiles and, in slices of up to 131,072 elements,
+ * the same bits. */
 int mfp_matrix_create_scoo(int value_type, uint32_t rows, uint32_t cols, uint32_t nnz,
                            const mfp_scoo_params *params, const uint32_t *c_index,
                            const uint32_t *r_index, const uint32_t *slices_ptr,

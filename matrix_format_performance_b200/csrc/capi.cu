@@ -249,9 +249,8 @@ constexpr uint32_t kDefaultAssist = 64;
 // touches: one or two passes), bits 16-23 with FP64 values (at least half).
 // Fewer lanes let a warp span more rows, whose x gathers share cache lines, but
 // a pass should read whole 128-byte lines of the values: the FP32 banded matrix
-// with 8 lanes (128 bytes) ran 378 us on 8M rows and with 4 lanes 485, which
-// fetch a line's halves at different times; in FP64 (4M rows) 4 lanes ran 274 us
-// and 8 lanes 298.  *regular = elements in blocks without either.
+// (8M rows) took 28% longer with 4 lanes, which fetch a line's halves at different
+// times, than with 8 (128 bytes); in FP64 (4M rows) 8 lanes took 9% longer than 4.  *regular = elements in blocks without either.
 // (row_blocks_regular: the share of that from every n-th block, to tell a
 // power-law matrix without reading all of its row_ptr.)
 bool row_blocks_regular(uint32_t rows, const uint32_t *rp) {
@@ -293,8 +292,8 @@ std::vector<uint4> row_block_info(uint32_t rows, const uint32_t *rp, uint32_t lo
 // (each extra piece adds a CTA-wide FP64 reduction and the combine).  But a
 // piece of 50,000 elements takes its CTA 30 to 70 us, which is longer than a
 // small matrix's whole product should: pieces of nnz / 512 elements (at least
-// 2,048) keep a piece to a fraction of it.  Power-law 100k rows FP64 31 -> 12.6
-// us, 300k rows FP32 31.5 -> 17.9, 1M rows FP64 74 -> 50, 4M rows unchanged;
+// 2,048) keep a piece to a fraction of it.  Power-law 100k rows FP64 52.7 -> 12.3
+// us, 300k rows FP32 38.1 -> 19.3, 1M rows FP64 76.0 -> 53.5, 4M rows unchanged;
 // nnz / 1024 and nnz / 4096 were 0-4 us slower from 300k rows on.
 constexpr uint32_t kDefaultPiece = 65536, kMinPiece = 2048, kPieceShare = 512;
 // Bytes of the counters at the head of a call's long-row scratch.
@@ -440,13 +439,13 @@ static int csr_plan_create(int value_type, uint32_t rows, uint32_t cols, uint32_
   // the others in the CSR-Adaptive bins beside them (two launches).  Batches of 40
   // to 64 uneven matrices, bins alone -> both, FP32: from 64M elements 228 -> 218 us
   // (78M), 232 -> 223 (71M), 208 -> 208 (69M), but between 92 -> 97 (35M), 128 -> 137
-  // (49M) and 178 -> 169 (53M) below; FP64 172 -> 181 (47M), 353 -> 363 (83M).  B200 against the row blocks / bins / warp
-  // tiles, inputs changing from pass to pass: banded 8M rows FP32 scalar 400 ->
-  // 361 us, vector 539 -> 341, 4M rows FP64 scalar 351 -> 275; 27-point 128^3 FP32
-  // scalar 121 -> 107, Adaptive 135 -> 97, 101^3 FP64 vector 96 -> 73; 5-point
-  // 1000^2 FP64 vector 27.5 -> 21; uniform 500k rows FP32 91 -> 79.  A power-law
-  // matrix has a row above 64 elements in nine blocks of ten and keeps its
-  // kernels.
+  // (49M) and 178 -> 169 (53M) below; FP64 172 -> 181 (47M), 353 -> 363 (83M).
+  // B200 against the row blocks / bins / warp tiles, inputs changing from pass to
+  // pass: banded 8M rows FP32 scalar 431 -> 406 us, vector 544 -> 367, 4M rows FP64
+  // scalar 335 -> 282; 27-point 128^3 FP32 scalar 121 -> 114, Adaptive 123 -> 102,
+  // 101^3 FP64 vector 96.7 -> 79.4; 5-point 1000^2 FP64 vector 27.0 -> 22.5; 4 to 64
+  // elements, 500k rows FP32 90 -> 79.  A power-law matrix has a row above 64
+  // elements in nine blocks of ten and keeps its kernels.
   std::vector<uint4> blk;
   if (MFP_CSR_DIRECT && automatic && nnz && row_blocks_regular(rows, rp)) {
     uint64_t regular = 0;
@@ -1590,13 +1589,13 @@ int scoo_attach_windows(mfp_matrix *m, const std::vector<uint32_t> &win, const u
 // Whether a row-ordered SCOO handle runs its slices' warp tiles as independent
 // warps (scoo_tile_kernel) instead of one CTA per slice (scoo_kernel):
 //  - when the heaviest slice holds more than twice the mean, which that
-//    slice's CTA would work through alone (B200: power-law, 50k rows FP32 49.7
-//    -> 13.7 us, 1M rows FP64 107 -> 59 us, 4M rows FP32 184 -> 170 us);
+//    slice's CTA would work through alone (B200: power-law, 50k rows FP32 48 ->
+//    12.1 us, 1M rows FP64 110 -> 59.6 us, 4M rows FP32 178 -> 170 us);
 //  - when there is work for the whole chip, and the slices are fewer than four
 //    per SM or so short (under 16 tiles) that their CTA's
 //    rounds of 8 tiles, barriers and x window weigh (27-point 40^3, 148
-//    slices, FP32 17.8 -> 12.1 us; 5-point 1400^2 FP64, 10 tiles each, 79.8 ->
-//    49.9 us; 1000^2 FP32 27.2 -> 22.6 us).
+//    slices, FP32 17.7 -> 12.2 us; 5-point 1400^2 FP64, 10 tiles each, 79.8 ->
+//    50.2 us; 1000^2 FP32 27.2 -> 22.6 us).
 // Long balanced slices stay with the one launch (27-point 128^3 122 us against
 // 139, banded 2M rows 118 against 128, 400k rows 28.5 against 31.4: no tile table
 // to wait for), and so do

@@ -530,12 +530,14 @@ __global__ void __launch_bounds__(kThreads) scoo_windows_kernel(uint32_t nnz, co
 // payload, a stable LSD radix sort when the input is not already in CSR
 // order, then row_ptr from the row boundaries of the sorted rows.
 //
-// One launch per digit.  A pass reads and writes 12 bytes per FP32 element (24
-// in all); the histograms of every digit come from one read of the ids before
-// the passes, the first pass reads the triplets themselves and the last one
-// writes the CSR arrays.  B200, 15.1M elements of 2M rows (42 key bits), FP32:
-// 920 us: 74 for the histograms and 150 a pass (2.4 TB/s; shared memory at 56%
-// and instruction issue at 50% of their rates, 32 warps per SM).  It was 1,340
+// One launch per digit, as in the published one-sweep radix sort (Adinets and
+// Merrill, 2022), with the decoupled look-back of Merrill and Garland (2016).  A
+// pass reads and writes 12 bytes per FP32 element (24 in all); the histograms of
+// every digit come from one read of the ids before the passes, the first pass
+// reads the triplets themselves and the last one writes the CSR arrays.  B200,
+// 15.1M elements of 2M rows (42 key bits), FP32: 894 us: 75 for the
+// histograms and 145 a pass (2.4 TB/s; shared memory at 54% and instruction issue
+// at 53% of their rates, 31 warps per SM).  It was 1,340
 // us with five launches per 8-bit digit (histogram 39 us, scans 12, scatter
 // 137, whose __match_any_sync kept one pipe 74% busy), 130 for making the keys
 // and 100 for splitting them.  Equal digits found with a shared-memory atomicOr

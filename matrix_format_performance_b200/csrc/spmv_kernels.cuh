@@ -7,6 +7,8 @@
 // same name:
 //   CSR scalar    one thread sums one row, in CSR order
 //                 (gpu/gpu_matrix_multiplier.cu:22-43)
+//   CSR, short    any CSR algorithm on blocks of short rows: lane groups read the
+//   rows          rows straight from global memory (csr_direct_kernel)
 //   CSR vector    a group of 2..32 lanes per row, lane-strided + shuffle tree
 //                 (gpu/gpu_matrix_multiplier.cu:331-362, gpu/reduce.cuh)
 //   CSR-Adaptive  host-built row bins; many-row bins reduce from shared
@@ -1024,9 +1026,10 @@ __global__ void __launch_bounds__(kBlock, sizeof(T) == 4 ? (ALGO != 1 ? MFP_CSR_
 // Staging the products through shared memory instead, and the 8-element lane
 // groups of the warp-tile kernel, spend the L1 data path on it: 10.6 wavefronts
 // per 32 nonzeros on the banded matrix, 65% of the L1 rate with DRAM at 79%.
-// Here the banded matrix (8M rows, FP32: 341 us summed by trees, 361 in order) is
-// at 100% and 95% of the DRAM rate; the 27-point stencil (128^3: 97 and 107 us)
-// spends its L1 wavefronts on the gathers, 8 cache lines for 32 lanes.
+// Here the banded matrix (8M rows, FP32: 367 us summed by trees, 406 in order,
+// inputs changing from pass to pass) runs at 94% and 85% of the copy rate, its L1
+// data path at 61% and 66%; the 27-point stencil (128^3: 102 and 114 us) spends
+// its L1 wavefronts on the gathers, 8 cache lines for 32 lanes (FP64 101^3: 74%).
 // ---------------------------------------------------------------------------
 template <typename T>
 struct row_quad {
@@ -1112,7 +1115,7 @@ __device__ __forceinline__ void csr_rows_direct(const csr_args<T> &A, uint64_t p
 
 // CTAs per SM the kernel is register-limited to (FP32, FP64).  Warps in flight
 // count for more than loads per warp: with two rounds of rows in flight per warp
-// at 5 CTAs (FP64: 4) the banded matrix took 378 us, here 361.
+// at 5 CTAs (FP64: 4) the banded matrix took 5% longer.
 #ifndef MFP_DIRECT_MINBLOCKS
 #define MFP_DIRECT_MINBLOCKS 8
 #endif
@@ -1961,11 +1964,11 @@ __global__ void __launch_bounds__(kBlock, sizeof(T) == 4 ? MFP_SCOO_MINBLOCKS : 
 // (from the slice's first element, rounded down to 8) as independent warps,
 // taken from a tile table, then a fix-up of the rows that cross tiles.  The
 // tiles, their reduction and the order of a crossing row's partial sums are
-// scoo_kernel's, so the bits are too; what changes is that a slice is no
-// longer one CTA's work.  One CTA per slice is bound by the heaviest slice: a
-// 1M-row power-law matrix (FP64, mean 7.5, rows up to 50,000) has a slice of
-// 200 tiles among slices of 15, and took 107 us there, 59 us here (the chip's
-// random x gathers are what is left).  At 8 CTAs per SM the FP32 kernel spills
+// scoo_kernel's, so the bits are too (up to kScooTiles tiles a slice); what
+// changes is that a slice is no longer one CTA's work.  One CTA per slice is bound
+// by the heaviest slice: a 1M-row power-law matrix (FP64, mean 7.5, rows up to
+// 50,000) has a slice of 200 tiles among slices of 15, and took 110 us there, 60 us
+// here (54 and 11 under ncu; the chip's random x gathers are what is left).  At 8 CTAs per SM the FP32 kernel spills
 // (4M-row power-law 176 us against 170 at 6).
 // ---------------------------------------------------------------------------
 struct scoo_tile {
