@@ -11,7 +11,7 @@ pattern (mfp_selector_features):
   configurations the matrix admits; with verify=k it times the k smallest
   on the matrix (k of the 28 configurations) and takes the fastest, which
   absorbs the network's near-ties (on the measured held-out set: within 5%
-  of the best for 84% of the matrices from the prediction alone, 95.5% with
+  of the best for 80.5% of the matrices from the prediction alone, 96.5% with
   the three best predictions timed);
 - **training**: on the engine's own kernels (mfp_mlp_forward /
   mfp_mlp_backward / mfp_mlp_adam), against times the engine measured on
